@@ -15,6 +15,7 @@ struct bdda_plan {
   size_t tw64_off[3];   // double2[M]: exp(-2 pi i k / M)
   size_t tw32_off[3];   // float2[M]: the same, rounded
   size_t rev_off[3];    // int32[M]: stored position -> frequency index
+  size_t pos_off[3];    // uint16[M]: frequency index -> stored position
   size_t err_off;       // uint32: bounded waits of the plan's kernels that gave up
   size_t table_bytes;
   std::vector<unsigned char> host_tables;

@@ -1,0 +1,14 @@
+// Two-register-stage kernels, complex64: X passes, lengths up to 128.
+#include "bdda_line.cuh"
+
+namespace bdda {
+
+#define BDDA_LINE_ENTRY(MM) {MM, conv_entry<float2, MM>()},
+static const LineKernel kTable[] = {BDDA_LINE_SHORT(BDDA_LINE_ENTRY)};
+
+const LineKernel* line_conv_c64_a(int* n) {
+  *n = (int)(sizeof(kTable) / sizeof(kTable[0]));
+  return kTable;
+}
+
+}  // namespace bdda

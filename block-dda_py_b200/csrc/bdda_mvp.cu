@@ -192,6 +192,63 @@ static std::vector<int> fixed_variants(int prec, int kind, int lt, const AxisFFT
   return out;
 }
 
+#define BDDA_LINE_ROW(PREC, KIND, NAME) {PREC, KIND, &NAME},
+static const struct { int prec, kind; LineTableFn table; } kLineTables[] = {BDDA_LINE_TABLES(BDDA_LINE_ROW)};
+#undef BDDA_LINE_ROW
+
+// Long axes (M >= 192) with complex128 kernels specialised for their radix
+// sequence keep those: block BiCGSTAB amplifies a difference in a product's last
+// bits up to 1e9-fold in S_bk on particles of that size, the
+// two-register-stage kernels gain only 4 % there (192 x 224 x 350, L = 64:
+// 37.0 against 38.6 ms a product), and so such solutions stay the same bits.
+// The specialised kernel taken is the one with the widest TMA-filled tile
+// (52.8 ms with the first one compiled).
+static const FixedKernel* fixed_long(int kind, const AxisFFT& ax) {
+  if (!g_use_fixed || ax.M < 192 || ax.nst > 4) return nullptr;
+  const FixedKernel* best = nullptr;
+  for (int t = 0; t < kFixedTables; ++t) {
+    int n = 0;
+    const FixedKernel* tab = fixed_table(t, &n);
+    for (int i = 0; i < n; ++i) {
+      const FixedKernel& f = tab[i];
+      bool same = f.prec == 0 && f.kind == kind && f.variant < 2048;
+      for (int s = 0; s < 4; ++s) same = same && f.r[s] == (s < ax.nst ? ax.rad[s] : 1);
+      if (!same) continue;
+      const bool tma = f.variant & 1024, btma = best && (best->variant & 1024);
+      if (!best || (tma && (!btma || f.lt > best->lt))) best = &f;
+    }
+  }
+  return best;
+}
+
+// Two-register-stage kernel of a pass (bdda_line.cuh), or null: the length must
+// have a split, and the rows a product reads (forward), writes (inverse) or
+// both (X) lie in the first half of the pencil, as on any grid M >= 2 N.
+static LineLaunchFn line_find(int prec, int kind, const PassArgs& a) {
+  if (!g_use_fixed || !a.pos || a.ax.M % 2) return nullptr;
+  const int M = a.ax.M;
+  int want = kind;
+  if (kind == K_FWD) {
+    if (a.n_out != M) return nullptr;
+    if (2 * a.n_in > M) {
+      if (a.n_in != M || a.cell_map) return nullptr;
+      want = 3;
+    }
+  } else if (kind == K_INV) {
+    if (a.n_in != M || 2 * a.n_out > M) return nullptr;
+  } else {
+    if (2 * a.n_in > M || 2 * a.n_out > M || a.src_p1 != a.C || a.dst_p1 != a.C || a.src_p0 != a.dst_p0) return nullptr;
+  }
+  for (const auto& t : kLineTables) {
+    if (t.prec != prec || t.kind != want) continue;
+    int n = 0;
+    const LineKernel* k = t.table(&n);
+    for (int i = 0; i < n; ++i)
+      if (k[i].M == M && k[i].fn) return k[i].fn;
+  }
+  return nullptr;
+}
+
 // Generic kernels: variant -1 with the first stage's global loads, -2 with the
 // TMA-filled tile; with no choice made (variant 0) and no specialised kernel
 // for the radix sequence, the TMA-filled one where the pass allows it.
@@ -200,6 +257,12 @@ static int launch_pass(const PassArgs& a, int64_t P0, int lt, cudaStream_t st) {
   int variant = 0;
   if (!a.green) {
     variant = pass_tune(prec_of<T>(), KIND, a.ax.M, a.L).variant;
+    if (variant == 0) {
+      const FixedKernel* f = prec_of<T>() == 0 ? fixed_long(KIND, a.ax) : nullptr;
+      if (f) return f->fn(a, P0, st);
+      const LineLaunchFn line = line_find(prec_of<T>(), KIND, a);
+      if (line) return line(a, P0, st);
+    }
     FixedLaunchFn f = fixed_find(prec_of<T>(), KIND, lt, a.ax, variant, pair_ok(a));
     if (f) return f(a, P0, st);
   }
@@ -240,6 +303,7 @@ void mvp_pass_args(const bdda_plan* plan, int L, const T* ghat, const int32_t* c
     PassArgs& q = a[0];
     q = b;
     q.ax = plan->ax[2]; q.tw = table_ptr<T>(plan, TwOff<T>::get(plan, 2));
+    q.pos = table_ptr<uint16_t>(plan, plan->pos_off[2]);
     q.n_in = (int)Nz; q.n_out = (int)Mz; q.P1 = (int)Ny;
     q.cell_map = cell_map; q.cell_p0 = Ny * Nz; q.cell_p1 = Nz;
     q.S = src;
@@ -249,6 +313,7 @@ void mvp_pass_args(const bdda_plan* plan, int L, const T* ghat, const int32_t* c
   }
   PassArgs ay = b;  // Y and Y^-1 share the pencil geometry
   ay.ax = plan->ax[1]; ay.tw = table_ptr<T>(plan, TwOff<T>::get(plan, 1));
+  ay.pos = table_ptr<uint16_t>(plan, plan->pos_off[1]);
   ay.P1 = (int)Mz; ay.src = F; ay.dst = F;
   ay.src_p0 = ay.dst_p0 = My * Mz * C; ay.src_p1 = ay.dst_p1 = C; ay.src_row = ay.dst_row = Mz * C;
   a[1] = ay;
@@ -258,6 +323,7 @@ void mvp_pass_args(const bdda_plan* plan, int L, const T* ghat, const int32_t* c
     PassArgs& q = a[2];
     q = b;
     q.ax = plan->ax[0]; q.tw = table_ptr<T>(plan, TwOff<T>::get(plan, 0));
+    q.pos = table_ptr<uint16_t>(plan, plan->pos_off[0]);
     q.n_in = (int)Nx; q.n_out = (int)Nx; q.P1 = (int)Mz;
     q.src = F; q.dst = F;
     q.src_p0 = q.dst_p0 = Mz * C; q.src_p1 = q.dst_p1 = C; q.src_row = q.dst_row = My * Mz * C;
@@ -271,6 +337,7 @@ void mvp_pass_args(const bdda_plan* plan, int L, const T* ghat, const int32_t* c
     PassArgs& q = a[4];
     q = b;
     q.ax = plan->ax[2]; q.tw = table_ptr<T>(plan, TwOff<T>::get(plan, 2));
+    q.pos = table_ptr<uint16_t>(plan, plan->pos_off[2]);
     q.n_in = (int)Mz; q.n_out = (int)Nz; q.P1 = (int)Ny;
     q.src = F; q.src_p0 = My * Mz * C; q.src_p1 = Mz * C; q.src_row = C;
     q.cell_map = cell_map; q.cell_p0 = Ny * Nz; q.cell_p1 = Nz;
@@ -361,6 +428,13 @@ static int autotune_impl(const bdda_plan* p, int L, const T* ghat, const int32_t
       Key key;
       key.kind = pass_kind[q];
       key.axis = pass_axis[q];
+      if (line_find(prec, key.kind, pa[q])) {   // variant 0, at any tile width
+        for (int lt : {8, 4, 2})
+          if (pencil_smem<T>(M, lt, key.kind) <= 227 * 1024) {
+            key.cand.push_back({prec, key.kind, M, L, lt, 0});
+            break;
+          }
+      }
       for (int lt : {16, 8, 4, 2}) {
         if (lt > 2 && lt / 2 >= L) continue;
         if (pencil_smem<T>(M, lt, key.kind) > 227 * 1024) continue;
@@ -675,6 +749,7 @@ int bdda_plan_create(const int n[3], const int m[3], bdda_plan** out) {
     p->tw64_off[a] = off; off = align256(off + (size_t)M * sizeof(double2));
     p->tw32_off[a] = off; off = align256(off + (size_t)M * sizeof(float2));
     p->rev_off[a] = off;  off = align256(off + (size_t)M * sizeof(int32_t));
+    p->pos_off[a] = off;  off = align256(off + (size_t)M * sizeof(uint16_t));
   }
   p->err_off = off; off = align256(off + sizeof(uint32_t));
   p->table_bytes = off;
@@ -685,6 +760,7 @@ int bdda_plan_create(const int n[3], const int m[3], bdda_plan** out) {
     double2* t64 = reinterpret_cast<double2*>(p->host_tables.data() + p->tw64_off[a]);
     float2* t32 = reinterpret_cast<float2*>(p->host_tables.data() + p->tw32_off[a]);
     int32_t* rev = reinterpret_cast<int32_t*>(p->host_tables.data() + p->rev_off[a]);
+    uint16_t* pos = reinterpret_cast<uint16_t*>(p->host_tables.data() + p->pos_off[a]);
     const long double twopi = 6.283185307179586476925286766559005768L;
     for (int k = 0; k < M; ++k) {
       const long double ang = twopi * (long double)k / (long double)M;
@@ -702,6 +778,7 @@ int bdda_plan_create(const int n[3], const int m[3], bdda_plan** out) {
         mult *= ax.rad[s2];
       }
       rev[k] = f;
+      pos[f] = (uint16_t)k;
     }
   }
   *out = p;
@@ -775,21 +852,28 @@ int bdda_green_build(const bdda_plan* p, double lf, double k, void* ghat, void* 
     a.dst = G; a.dst_p0 = My * Mz * 6; a.dst_p1 = Mz * 6; a.dst_row = 6;
     BDDA_TRY((launch_lt<double2, K_FWD, 2>(a, Mx, st)));
   }
+  // every row of these pencils holds data
+  auto forward = [&](const PassArgs& a, int64_t P0, int kind) -> int {
+    const LineLaunchFn line = fixed_long(kind, a.ax) ? nullptr : line_find(BDDA_C128, K_FWD, a);
+    return line ? line(a, P0, st) : launch_lt<double2, K_FWD, 2>(a, P0, st);
+  };
   {  // forward y
     PassArgs a = b;
     a.ax = p->ax[1]; a.tw = table_ptr<double2>(p, p->tw64_off[1]);
+    a.pos = table_ptr<uint16_t>(p, p->pos_off[1]);
     a.n_in = a.n_out = (int)My; a.P1 = (int)Mz;
     a.src = G; a.dst = G;
     a.src_p0 = a.dst_p0 = My * Mz * 6; a.src_p1 = a.dst_p1 = 6; a.src_row = a.dst_row = Mz * 6;
-    BDDA_TRY((launch_lt<double2, K_FWD, 2>(a, Mx, st)));
+    BDDA_TRY(forward(a, Mx, K_FWD));
   }
   {  // forward x into the x-pencil-major spectrum
     PassArgs a = b;
     a.ax = p->ax[0]; a.tw = table_ptr<double2>(p, p->tw64_off[0]);
+    a.pos = table_ptr<uint16_t>(p, p->pos_off[0]);
     a.n_in = a.n_out = (int)Mx; a.P1 = (int)Mz;
     a.src = G; a.src_p0 = Mz * 6; a.src_p1 = 6; a.src_row = My * Mz * 6;
     a.dst = ghat; a.dst_p0 = Mz * Mx * 6; a.dst_p1 = Mx * 6; a.dst_row = 6;
-    BDDA_TRY((launch_lt<double2, K_FWD, 2>(a, My, st)));
+    BDDA_TRY(forward(a, My, K_CONV));
   }
   return BDDA_OK;
 }

@@ -33,6 +33,7 @@ struct PassArgs {
   const void* src;
   void* dst;
   const void* tw;       // this axis' twiddles, M entries
+  const uint16_t* pos;  // this axis' frequency -> stored position table, M entries
   const int32_t* cell_map;   // K_FWD: gather S through it; K_INV: scatter with the epilogue
   int64_t cell_p0, cell_p1;
   const void* S;
@@ -558,6 +559,27 @@ struct FixedKernel {
   FixedLaunchFn fn;
   int pair;            // 1: column-pair jobs (needs even L and 16-byte aligned fields)
 };
+// Two-register-stage kernels of one axis length (bdda_line.cuh), tables by
+// precision, pass kind (3: a forward pass whose M rows all hold data) and
+// length range.
+typedef int (*LineLaunchFn)(const PassArgs& a, int64_t P0, cudaStream_t st);
+struct LineKernel {
+  int M;
+  LineLaunchFn fn;
+};
+typedef const LineKernel* (*LineTableFn)(int* n);
+#define BDDA_LINE_TABLES(F)                                                                            \
+  F(0, K_FWD, line_fwd_c128_a) F(0, K_FWD, line_fwd_c128_b) F(0, K_FWD, line_fwd_c128_c)               \
+  F(0, K_INV, line_inv_c128_a) F(0, K_INV, line_inv_c128_b) F(0, K_INV, line_inv_c128_c)               \
+  F(0, K_CONV, line_conv_c128_a) F(0, K_CONV, line_conv_c128_b)                                        \
+  F(1, K_FWD, line_fwd_c64_a) F(1, K_FWD, line_fwd_c64_b) F(1, K_FWD, line_fwd_c64_c)                  \
+  F(1, K_INV, line_inv_c64_a) F(1, K_INV, line_inv_c64_b) F(1, K_INV, line_inv_c64_c)                  \
+  F(1, K_CONV, line_conv_c64_a) F(1, K_CONV, line_conv_c64_b)                                          \
+  F(0, 3, line_full_c128_a) F(0, 3, line_full_c128_b) F(0, 3, line_full_c128_c)
+#define BDDA_LINE_DECL(PREC, KIND, NAME) const LineKernel* NAME(int* n);
+BDDA_LINE_TABLES(BDDA_LINE_DECL)
+#undef BDDA_LINE_DECL
+
 const FixedKernel* fixed_table_a(int* n);
 const FixedKernel* fixed_table_b(int* n);
 const FixedKernel* fixed_table_c(int* n);

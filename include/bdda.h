@@ -97,7 +97,9 @@ int bdda_tune_set(int prec, int kind, size_t smem_budget, int threads);
 int bdda_tune_get(int prec, int kind, size_t* smem_budget, int* threads);
 /* Per-pass launch choice for passes of (prec, kind) over an axis of length M
  * at block width L: column tile width lt (2, 4, 8, 16; 0 = the smem_budget rule)
- * and kernel variant (0 = the first specialised kernel compiled for the radix
+ * and kernel variant (0 = the library's choice: the two-register-stage kernel
+ * of the axis length (even 7-smooth lengths from 16 to 540), except where a
+ * complex128 axis of at least 192 points has kernels specialised for its radix
  * sequence; k in 1..8 = the one of 256 threads compiled for k resident CTAs
  * per SM; k + 16 * (threads / 32) = the one of that CTA size; 512 + either
  * = a complex64 kernel whose jobs take two adjacent columns, used when L is
