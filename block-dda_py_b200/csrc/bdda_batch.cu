@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(256) batch_gram_kernel(const GramArgs* args, c
 __global__ void batch_gram_reduce_kernel(const GramArgs* args, const ProbDev* pd, const int* flags, int width) {
   const int p = blockIdx.y;
   if (!flags[p]) return;
-  gram_reduce_body(args[p].partial, pd[p].nblk, width, pd[p].sp.g2, blockIdx.x * blockDim.x + threadIdx.x);
+  gram_reduce_body(args[p].partial, pd[p].nblk, width, pd[p].sp.g2, blockIdx.x * kReduceOut);
 }
 
 template <typename T, typename A, int L>
@@ -688,7 +688,7 @@ struct Engine {
       batch_gram_kernel<T, true, LL, 2><<<cap(gram_grid[1], upper[kClsBlas]), 256, gram_smem[1], st>>>(g, pd, list);
     BDDA_CUDA_TRY(cudaGetLastError());
     const int width = nb * LL * LL;
-    batch_gram_reduce_kernel<<<dim3((width + 255) / 256, nprob), 256, 0, st>>>(g, pd, flags, width);
+    batch_gram_reduce_kernel<<<dim3((width + kReduceOut - 1) / kReduceOut, nprob), 256, 0, st>>>(g, pd, flags, width);
     BDDA_CUDA_TRY(cudaGetLastError());
     count(2);
     return BDDA_OK;
@@ -955,7 +955,7 @@ int batch_run(const bdda_batch_problem* pr, int nprob, int mode, int L, double t
   e32.list.cnt = l0.cnt + (size_t)kNCls * np;   // the lists share their buffers: the last build counts
   e32.pd = dpd;
   const int gp = (nprob + 255) / 256;
-  const size_t sm2 = (size_t)2 * L * L * sizeof(double2);
+  const size_t sm2 = (size_t)small_elems(L, 2) * sizeof(double2);
   BDDA_CUDA_TRY(cudaFuncSetAttribute(batch_alpha_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2));
   BDDA_CUDA_TRY(cudaFuncSetAttribute(batch_zeta_beta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2));
 

@@ -11,18 +11,41 @@ namespace bdda {
 // L-specialised Gram / update kernels on (tests switch them off to compare).
 static int g_fixed_blas = 1;
 
-// ---- Gram: G_k[i][j] = sum_r op(A[r][i]) B_k[r][j] ---------------------------
-template <typename T, bool CONJ, int TM, int NB>
+// ---- Gram: G_k[i][j] = sum_r op(A[r][i]) B_k[r][j], any L <= 64 ---------------
+// The L x L tile is padded to LP = NT TM columns and computed by NT x NT
+// threads with TM x TM elements each (rows ty + NT i, columns tx + NT j, so a warp
+// reads consecutive words); narrow blocks leave room for GROUPS = 256 / NT^2
+// such thread grids, which take the rows of a chunk in turn and are added at
+// the end.  Chunks are double-buffered with cp.async.  The kernel before
+// (one thread grid whatever L, no prefetch) ran L = 1 with one thread of 256
+// busy: 97 us for 3 x 105,000 rows and two products, 9 us now.
+template <int BYTES>
+__device__ __forceinline__ void cp_async_elem(void* smem, const void* gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+
+template <int NT, int TM> struct GramShape {
+  static constexpr int LP = NT * TM, GROUPS = 256 / (NT * NT);
+  // rows per chunk: 512 / LP for narrow blocks, 16 for wide ones
+  static constexpr int RCH = 512 / LP > 16 ? 512 / LP : 16;
+};
+
+template <typename T, bool CONJ, int NT, int TM, int NB>
 __global__ void __launch_bounds__(256) gram_kernel(GramArgs g) {
-  constexpr int RCH = 16;
-  const int L = g.L;
-  const int nt = (L + TM - 1) / TM;
-  const int t = threadIdx.x;
-  const int ty = t / nt, tx = t - ty * nt;
-  const bool active = ty < nt;
-  extern __shared__ double2 gsh[];
-  double2* sA = gsh;
-  double2* sB = gsh + RCH * L;
+  typedef GramShape<NT, TM> S;
+  constexpr int LP = S::LP, GROUPS = S::GROUPS, RCH = S::RCH, CH = RCH * LP;
+  extern __shared__ __align__(16) unsigned char gsh[];
+  T* buf = reinterpret_cast<T*>(gsh);   // [2][1 + NB][RCH][LP]
+  const int L = g.L, t = threadIdx.x;
+  const int grp = t / (NT * NT), tt = t - grp * (NT * NT), ty = tt / NT, tx = tt - ty * NT;
+  const float by_l = 1.f / L;
+  T zero;
+  zero.x = 0;
+  zero.y = 0;
+  for (int e = t; e < 2 * (1 + NB) * CH; e += 256) buf[e] = zero;   // the columns at or past L stay zero
+  __syncthreads();
   double2 acc[NB][TM][TM];
 #pragma unroll
   for (int k = 0; k < NB; ++k)
@@ -30,66 +53,87 @@ __global__ void __launch_bounds__(256) gram_kernel(GramArgs g) {
     for (int i = 0; i < TM; ++i)
 #pragma unroll
       for (int j = 0; j < TM; ++j) acc[k][i][j] = make_double2(0.0, 0.0);
-  const int64_t chunk = (g.n + gridDim.x - 1) / gridDim.x;
-  const int64_t r0 = blockIdx.x * chunk;
-  const int64_t r1 = min(g.n, r0 + chunk);
-  const T* A = static_cast<const T*>(g.A);
-  for (int64_t rb = r0; rb < r1; rb += RCH) {
-    const int rows = (int)min((int64_t)RCH, r1 - rb);
-    for (int e = t; e < RCH * L; e += blockDim.x) {
-      const int r = e / L;
-      double2 v = make_double2(0.0, 0.0);
-      if (r < rows) {
-        v = ld_as<double2>(A, rb * L + e);
-        if (CONJ) v.y = -v.y;
+  const int64_t nchunks = (g.n + RCH - 1) / RCH;
+  const int64_t per = (nchunks + gridDim.x - 1) / gridDim.x;
+  const int64_t c0 = blockIdx.x * per, c1 = min(nchunks, c0 + per);
+  const T* src[1 + NB];
+  src[0] = static_cast<const T*>(g.A);
+#pragma unroll
+  for (int k = 0; k < NB; ++k) src[1 + k] = static_cast<const T*>(g.B[k]);
+  auto stage = [&](int64_t ck, int slot) {
+    const int64_t r0 = ck * RCH;
+    const int valid = (int)min((int64_t)RCH, g.n - r0) * L;
+    for (int e = t; e < RCH * L; e += 256) {
+      const int r = (int)((e + 0.5f) * by_l), c = e - r * L;
+#pragma unroll
+      for (int m = 0; m < 1 + NB; ++m) {
+        T* d = buf + (slot * (1 + NB) + m) * CH + r * LP + c;
+        if (e < valid) cp_async_elem<(int)sizeof(T)>(d, src[m] + r0 * L + e);
+        else *d = zero;
       }
-      sA[e] = v;
+    }
+  };
+  if (c0 < c1) stage(c0, 0);
+  cp_async_commit_g();
+  for (int64_t ck = c0; ck < c1; ++ck) {
+    const int slot = (int)((ck - c0) & 1);
+    if (ck + 1 < c1) stage(ck + 1, slot ^ 1);
+    cp_async_commit_g();
+    cp_async_wait_g<1>();
+    __syncthreads();
+    const T* sA = buf + slot * (1 + NB) * CH;
+#pragma unroll 2
+    for (int r = grp; r < RCH; r += GROUPS) {
+      double2 a[TM], b[NB][TM];
+#pragma unroll
+      for (int ii = 0; ii < TM; ++ii) {
+        a[ii] = to_d2(sA[r * LP + ty + NT * ii]);
+        if (CONJ) a[ii].y = -a[ii].y;
+      }
 #pragma unroll
       for (int k = 0; k < NB; ++k)
-        sB[k * RCH * L + e] = r < rows ? ld_as<double2>(static_cast<const T*>(g.B[k]), rb * L + e)
-                                       : make_double2(0.0, 0.0);
-    }
-    __syncthreads();
-    if (active) {
-      for (int r = 0; r < rows; ++r) {
-        double2 a[TM], b[NB][TM];
 #pragma unroll
-        for (int ii = 0; ii < TM; ++ii) {
-          const int i = ty * TM + ii;
-          a[ii] = i < L ? sA[r * L + i] : make_double2(0.0, 0.0);
-        }
+        for (int jj = 0; jj < TM; ++jj) b[k][jj] = to_d2(sA[(1 + k) * CH + r * LP + tx + NT * jj]);
 #pragma unroll
-        for (int k = 0; k < NB; ++k)
+      for (int k = 0; k < NB; ++k)
 #pragma unroll
-          for (int jj = 0; jj < TM; ++jj) {
-            const int j = tx * TM + jj;
-            b[k][jj] = j < L ? sB[k * RCH * L + r * L + j] : make_double2(0.0, 0.0);
-          }
+        for (int ii = 0; ii < TM; ++ii)
 #pragma unroll
-        for (int k = 0; k < NB; ++k)
-#pragma unroll
-          for (int ii = 0; ii < TM; ++ii)
-#pragma unroll
-            for (int jj = 0; jj < TM; ++jj) acc[k][ii][jj] = cfma(a[ii], b[k][jj], acc[k][ii][jj]);
-      }
+          for (int jj = 0; jj < TM; ++jj) acc[k][ii][jj] = cfma(a[ii], b[k][jj], acc[k][ii][jj]);
     }
     __syncthreads();
   }
-  if (active) {
+  cp_async_wait_g<0>();
+  double2* out = g.partial + (int64_t)blockIdx.x * NB * L * L;
+  if constexpr (GROUPS == 1) {
 #pragma unroll
     for (int k = 0; k < NB; ++k)
 #pragma unroll
       for (int ii = 0; ii < TM; ++ii)
 #pragma unroll
         for (int jj = 0; jj < TM; ++jj) {
-          const int i = ty * TM + ii, j = tx * TM + jj;
-          if (i < L && j < L) g.partial[(((int64_t)blockIdx.x * NB + k) * L + i) * L + j] = acc[k][ii][jj];
+          const int i = ty + NT * ii, j = tx + NT * jj;
+          if (i < L && j < L) out[(k * L + i) * L + j] = acc[k][ii][jj];
         }
+  } else {   // TM = 1: add the thread grids (rows of the chunk modulo GROUPS) in order
+    double2* red = reinterpret_cast<double2*>(gsh);   // [GROUPS][NB][NT][NT]: 512 elements at most
+#pragma unroll
+    for (int k = 0; k < NB; ++k) red[(grp * NB + k) * (NT * NT) + tt] = acc[k][0][0];
+    __syncthreads();
+    if (grp < NB && ty < L && tx < L) {
+      double2 s = make_double2(0.0, 0.0);
+      for (int q = 0; q < GROUPS; ++q) {
+        const double2 v = red[(q * NB + grp) * (NT * NT) + tt];
+        s.x += v.x;
+        s.y += v.y;
+      }
+      out[(grp * L + ty) * L + tx] = s;
+    }
   }
 }
 
 __global__ void gram_reduce_kernel(const double2* partial, int nblk, int width, double2* out) {
-  gram_reduce_body(partial, nblk, width, out, blockIdx.x * blockDim.x + threadIdx.x);
+  gram_reduce_body(partial, nblk, width, out, blockIdx.x * kReduceOut);
 }
 
 template <typename T, bool CONJ, int L, int NB>
@@ -112,31 +156,44 @@ static int gram_fixed(const GramArgs& g, double2* out, cudaStream_t st) {
   }
   BDDA_CUDA_TRY(cudaGetLastError());
   const int width = g.nB * L * L;
-  gram_reduce_kernel<<<(width + 255) / 256, 256, 0, st>>>(g.partial, kRedBlocks, width, out);
+  gram_reduce_kernel<<<(width + kReduceOut - 1) / kReduceOut, 256, 0, st>>>(g.partial, kRedBlocks, width, out);
   BDDA_CUDA_TRY(cudaGetLastError());
   count_launch(2);
   return BDDA_OK;
 }
 
-template <typename T, bool CONJ, int TM>
-static int gram_tm(const GramArgs& g, double2* out, cudaStream_t st) {
-  constexpr int RCH = 16;
-  const size_t smem = (size_t)RCH * g.L * (1 + g.nB) * sizeof(double2);
-  if (g.nB == 1) {
-    auto k = gram_kernel<T, CONJ, TM, 1>;
-    BDDA_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k<<<kRedBlocks, 256, smem, st>>>(g);
-  } else {
-    auto k = gram_kernel<T, CONJ, TM, 2>;
-    BDDA_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k<<<kRedBlocks, 256, smem, st>>>(g);
-  }
-  BDDA_CUDA_TRY(cudaGetLastError());
-  count_launch(2);
-  const int width = g.nB * g.L * g.L;
-  gram_reduce_kernel<<<(width + 255) / 256, 256, 0, st>>>(g.partial, kRedBlocks, width, out);
+template <typename T, bool CONJ, int NT, int TM, int NB>
+static int gram_launch(const GramArgs& g, cudaStream_t st) {
+  typedef GramShape<NT, TM> S;
+  const size_t stages = (size_t)2 * (1 + NB) * S::RCH * S::LP * sizeof(T), groups = (size_t)NB * 256 * sizeof(double2);
+  const size_t smem = stages > groups ? stages : groups;
+  auto k = gram_kernel<T, CONJ, NT, TM, NB>;
+  BDDA_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k<<<kRedBlocks, 256, smem, st>>>(g);
   BDDA_CUDA_TRY(cudaGetLastError());
   return BDDA_OK;
+}
+template <typename T, bool CONJ, int NT, int TM>
+static int gram_tm(const GramArgs& g, double2* out, cudaStream_t st) {
+  const int s = g.nB == 1 ? gram_launch<T, CONJ, NT, TM, 1>(g, st) : gram_launch<T, CONJ, NT, TM, 2>(g, st);
+  if (s != BDDA_OK) return s;
+  const int width = g.nB * g.L * g.L;
+  gram_reduce_kernel<<<(width + kReduceOut - 1) / kReduceOut, 256, 0, st>>>(g.partial, kRedBlocks, width, out);
+  BDDA_CUDA_TRY(cudaGetLastError());
+  count_launch(2);
+  return BDDA_OK;
+}
+// the smallest padded width that holds L
+template <typename T, bool CONJ>
+static int gram_any(const GramArgs& g, double2* out, cudaStream_t st) {
+  if (g.L == 1) return gram_tm<T, CONJ, 1, 1>(g, out, st);
+  if (g.L == 2) return gram_tm<T, CONJ, 2, 1>(g, out, st);
+  if (g.L <= 4) return gram_tm<T, CONJ, 4, 1>(g, out, st);
+  if (g.L <= 8) return gram_tm<T, CONJ, 8, 1>(g, out, st);
+  if (g.L <= 16) return gram_tm<T, CONJ, 16, 1>(g, out, st);
+  if (g.L <= 32) return gram_tm<T, CONJ, 16, 2>(g, out, st);
+  if (g.L <= 48) return gram_tm<T, CONJ, 16, 3>(g, out, st);
+  return gram_tm<T, CONJ, 16, 4>(g, out, st);
 }
 
 template <typename T>
@@ -150,32 +207,24 @@ int gram(const GramArgs& g, bool conj, double2* out, cudaStream_t st) {
     BDDA_GRAM_L(8) BDDA_GRAM_L(16) BDDA_GRAM_L(32) BDDA_GRAM_L(64)
 #undef BDDA_GRAM_L
   }
-  const int tm = g.L <= 16 ? 1 : (g.L <= 32 ? 2 : 4);
-  if (conj) {
-    if (tm == 1) return gram_tm<T, true, 1>(g, out, st);
-    if (tm == 2) return gram_tm<T, true, 2>(g, out, st);
-    return gram_tm<T, true, 4>(g, out, st);
-  }
-  if (tm == 1) return gram_tm<T, false, 1>(g, out, st);
-  if (tm == 2) return gram_tm<T, false, 2>(g, out, st);
-  return gram_tm<T, false, 4>(g, out, st);
+  return conj ? gram_any<T, true>(g, out, st) : gram_any<T, false>(g, out, st);
 }
 
-// ---- fused block update -------------------------------------------------------
+// ---- fused block update, any L <= 64 ----------------------------------------------
 // out = a0*Y0 + a1*Y1 + (X1 + c2*X2) M, arithmetic in A (double2 for c128,
-// float2 for c64 vectors), optional per-CTA partial of ||out||_F^2.
-template <typename T, typename A, int TN>
+// float2 for c64 vectors), optional per-CTA partial of ||out||_F^2.  NCG x NRG
+// threads; a thread owns two rows and the columns cg + NCG j (consecutive lanes
+// read consecutive words of M, padded to NCG TC columns).
+template <typename T, typename A, int NCG, int TC>
 __global__ void __launch_bounds__(256) update_kernel(UpdateArgs u) {
+  constexpr int LP = NCG * TC, NRG = 256 / NCG, TR = 2, RB = NRG * TR;
   const int L = u.L;
-  const int ncg = (L + TN - 1) / TN;
-  const int RCH = blockDim.x / ncg;
   extern __shared__ __align__(16) unsigned char ush[];
-  A* sM = reinterpret_cast<A*>(ush);
-  A* sX = sM + (u.M ? L * L : 0);
+  A* sM = reinterpret_cast<A*>(ush);           // [L][LP]
+  A* sX = sM + (u.M ? L * LP : 0);             // [RB][L]
   const int t = threadIdx.x;
-  const int rr = t / ncg, cg = t - rr * ncg;
-  const bool active = rr < RCH;
-  const A one = conv_acc<A>(make_double2(1.0, 0.0));
+  const int rg = t / NCG, cg = t - rg * NCG;
+  const A one = conv_acc<A>(make_double2(1.0, 0.0)), zero = conv_acc<A>(make_double2(0.0, 0.0));
   const A a0 = u.a0 ? conv_acc<A>(*u.a0) : one;
   const A a1 = u.a1 ? conv_acc<A>(*u.a1) : one;
   const A c2 = u.c2 ? conv_acc<A>(*u.c2) : one;
@@ -185,53 +234,62 @@ __global__ void __launch_bounds__(256) update_kernel(UpdateArgs u) {
   const T* X2 = static_cast<const T*>(u.X2);
   T* out = static_cast<T*>(u.out);
   if (u.M)
-    for (int e = t; e < L * L; e += blockDim.x) sM[e] = conv_acc<A>(u.M[e]);
+    for (int e = t; e < L * LP; e += 256) {
+      const int r = e / LP, c = e - r * LP;
+      sM[e] = c < L ? conv_acc<A>(u.M[r * L + c]) : zero;
+    }
   double nrm = 0.0;
-  for (int64_t rb = (int64_t)blockIdx.x * RCH; rb < u.n; rb += (int64_t)gridDim.x * RCH) {
+  for (int64_t rb = (int64_t)blockIdx.x * RB; rb < u.n; rb += (int64_t)gridDim.x * RB) {
     if (u.M) {
       __syncthreads();
-      for (int e = t; e < RCH * L; e += blockDim.x) {
-        const int64_t row = rb + e / L;
-        A v = conv_acc<A>(make_double2(0.0, 0.0));
-        if (row < u.n) {
+      const int64_t left = (u.n - rb) * L;
+      for (int e = t; e < RB * L; e += 256) {
+        A v = zero;
+        if (e < left) {
           v = ld_as<A>(X1, rb * L + e);
-          if (X2) {
-            const A w = ld_as<A>(X2, rb * L + e);
-            v = cfma(c2, w, v);
-          }
+          if (X2) v = cfma(c2, ld_as<A>(X2, rb * L + e), v);
         }
         sX[e] = v;
       }
       __syncthreads();
     }
-    const int64_t row = rb + rr;
-    if (active && row < u.n) {
-      A acc[TN];
+    A acc[TR][TC];
 #pragma unroll
-      for (int jj = 0; jj < TN; ++jj) {
-        const int j = cg * TN + jj;
-        acc[jj] = conv_acc<A>(make_double2(0.0, 0.0));
-        if (j < L) {
-          if (Y0) acc[jj] = cfma(a0, ld_as<A>(Y0, row * L + j), acc[jj]);
-          if (Y1) acc[jj] = cfma(a1, ld_as<A>(Y1, row * L + j), acc[jj]);
+    for (int ii = 0; ii < TR; ++ii) {
+      const int64_t row = rb + rg + NRG * ii;
+#pragma unroll
+      for (int jj = 0; jj < TC; ++jj) {
+        const int c = cg + NCG * jj;
+        acc[ii][jj] = zero;
+        if (row < u.n && c < L) {
+          if (Y0) acc[ii][jj] = cfma(a0, ld_as<A>(Y0, row * L + c), acc[ii][jj]);
+          if (Y1) acc[ii][jj] = cfma(a1, ld_as<A>(Y1, row * L + c), acc[ii][jj]);
         }
       }
-      if (u.M) {
-        for (int i = 0; i < L; ++i) {
-          const A x = sX[rr * L + i];
+    }
+    if (u.M) {
+#pragma unroll 4
+      for (int i = 0; i < L; ++i) {
+        A x[TR], m[TC];
 #pragma unroll
-          for (int jj = 0; jj < TN; ++jj) {
-            const int j = cg * TN + jj;
-            if (j < L) acc[jj] = cfma(x, sM[i * L + j], acc[jj]);
-          }
-        }
+        for (int ii = 0; ii < TR; ++ii) x[ii] = sX[(rg + NRG * ii) * L + i];
+#pragma unroll
+        for (int jj = 0; jj < TC; ++jj) m[jj] = sM[i * LP + cg + NCG * jj];
+#pragma unroll
+        for (int ii = 0; ii < TR; ++ii)
+#pragma unroll
+          for (int jj = 0; jj < TC; ++jj) acc[ii][jj] = cfma(x[ii], m[jj], acc[ii][jj]);
       }
+    }
 #pragma unroll
-      for (int jj = 0; jj < TN; ++jj) {
-        const int j = cg * TN + jj;
-        if (j < L) {
-          const T v = st_as<T>(acc[jj]);
-          out[row * L + j] = v;
+    for (int ii = 0; ii < TR; ++ii) {
+      const int64_t row = rb + rg + NRG * ii;
+#pragma unroll
+      for (int jj = 0; jj < TC; ++jj) {
+        const int c = cg + NCG * jj;
+        if (row < u.n && c < L) {
+          const T v = st_as<T>(acc[ii][jj]);
+          out[row * L + c] = v;
           const double2 vd = to_d2(v);
           nrm += vd.x * vd.x + vd.y * vd.y;
         }
@@ -242,6 +300,15 @@ __global__ void __launch_bounds__(256) update_kernel(UpdateArgs u) {
     const double s = block_sum(nrm);
     if (threadIdx.x == 0) u.norm_partial[blockIdx.x] = s;
   }
+}
+
+// CTAs of an update: kRedBlocks where the norm's partials are counted on,
+// else up to eight per SM (an update moves three or four vectors and little
+// else, so it needs the bytes in flight: 143 -> 107 us for 280,000 rows at L = 32).
+static int update_grid(const UpdateArgs& u, int rb) {
+  if (u.norm_partial) return kRedBlocks;
+  const int64_t b = (u.n + rb - 1) / rb;
+  return (int)(b < 1 ? 1 : b < 4 * kRedBlocks ? b : 4 * kRedBlocks);
 }
 
 template <typename T, typename A, int L>
@@ -257,20 +324,19 @@ static int update_fixed(const UpdateArgs& u, cudaStream_t st) {
   const size_t smem = u.M ? ((size_t)L * L + (size_t)RB * L) * sizeof(A) : 0;
   auto k = update_fixed_kernel<T, A, L>;
   BDDA_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k<<<kRedBlocks, 256, smem, st>>>(u);
+  k<<<update_grid(u, RB), 256, smem, st>>>(u);
   BDDA_CUDA_TRY(cudaGetLastError());
   count_launch();
   return BDDA_OK;
 }
 
-template <typename T, typename A, int TN>
+template <typename T, typename A, int NCG, int TC>
 static int update_tn(const UpdateArgs& u, cudaStream_t st) {
-  const int ncg = (u.L + TN - 1) / TN;
-  const int rch = 256 / ncg;
-  const size_t smem = ((u.M ? (size_t)u.L * u.L : 0) + (u.M ? (size_t)rch * u.L : 0)) * sizeof(A);
-  auto k = update_kernel<T, A, TN>;
+  constexpr int RB = 256 / NCG * 2;
+  const size_t smem = u.M ? ((size_t)u.L * NCG * TC + (size_t)RB * u.L) * sizeof(A) : 0;
+  auto k = update_kernel<T, A, NCG, TC>;
   BDDA_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k<<<kRedBlocks, 256, smem, st>>>(u);
+  k<<<update_grid(u, RB), 256, smem, st>>>(u);
   BDDA_CUDA_TRY(cudaGetLastError());
   count_launch();
   return BDDA_OK;
@@ -286,9 +352,14 @@ int update(const UpdateArgs& u, cudaStream_t st) {
     if (u.L == 16) return update_fixed<T, A, 16>(u, st);
     if (u.L == 8) return update_fixed<T, A, 8>(u, st);
   }
-  if (u.L >= 32) return update_tn<T, A, 4>(u, st);
-  if (u.L >= 16) return update_tn<T, A, 2>(u, st);
-  return update_tn<T, A, 1>(u, st);
+  if (u.L == 1) return update_tn<T, A, 1, 1>(u, st);
+  if (u.L == 2) return update_tn<T, A, 2, 1>(u, st);
+  if (u.L <= 4) return update_tn<T, A, 4, 1>(u, st);
+  if (u.L <= 8) return update_tn<T, A, 8, 1>(u, st);
+  if (u.L <= 16) return update_tn<T, A, 16, 1>(u, st);
+  if (u.L <= 32) return update_tn<T, A, 16, 2>(u, st);
+  if (u.L <= 48) return update_tn<T, A, 16, 3>(u, st);
+  return update_tn<T, A, 16, 4>(u, st);
 }
 
 template <typename T>

@@ -38,16 +38,28 @@ __device__ __forceinline__ float2 cfma(float2 a, float2 b, float2 c) {
   return make_float2(fmaf(a.x, b.x, fmaf(-a.y, b.y, c.x)), fmaf(a.x, b.y, fmaf(a.y, b.x, c.y)));
 }
 
-// Per-element reduction of gram partials: out[o] = sum_b partial[b][o].
-__device__ __forceinline__ void gram_reduce_body(const double2* partial, int nblk, int width, double2* out, int o) {
-  if (o >= width) return;
+// out[o] = sum_b partial[b][o], b ascending, for the kReduceOut elements from
+// o0: all partials are loaded at once (a CTA of 256 threads reads 128-byte runs),
+// then one thread per element adds them in order.  One thread loading and
+// adding partial after partial took 24 us for L = 8 (128 elements, 296
+// partials); 5 us now, the same sums.
+constexpr int kReduceOut = 8;
+__device__ __forceinline__ void gram_reduce_body(const double2* partial, int nblk, int width, double2* out, int o0) {
+  __shared__ double2 part[kRedBlocks * kReduceOut];
+  const int o = threadIdx.x % kReduceOut;
+  if (o0 + o < width)
+    for (int b = threadIdx.x / kReduceOut; b < nblk; b += 256 / kReduceOut)
+      part[b * kReduceOut + o] = partial[(int64_t)b * width + o0 + o];
+  __syncthreads();
+  if (threadIdx.x >= kReduceOut || o0 + o >= width) return;
   double2 s = make_double2(0.0, 0.0);
+#pragma unroll 8
   for (int b = 0; b < nblk; ++b) {
-    const double2 v = partial[(int64_t)b * width + o];
+    const double2 v = part[b * kReduceOut + o];
     s.x += v.x;
     s.y += v.y;
   }
-  out[o] = s;
+  out[o0 + o] = s;
 }
 
 // ---- Gram, specialised on L: split-K over row chunks, register tiles --------

@@ -80,7 +80,7 @@ int bdda_observables(int n_occ, int L, double k, double lf, int absorbing, const
   dda_epilogue_kernel<double2><<<kDdaObsBlocks, dda_epilogue_threads(L), dda_epilogue_smem(L), st>>>(
       a, static_cast<const double2*>(X), nullptr, static_cast<const double2*>(eper_r));
   BDDA_CUDA_TRY(cudaGetLastError());
-  observables_finalize_kernel<<<(L + 63) / 64, 64, 0, st>>>(a.partial, kDdaObsBlocks, L, k, absorbing, out);
+  observables_finalize_kernel<<<L, 256, 0, st>>>(a.partial, kDdaObsBlocks, L, k, absorbing, out);
   BDDA_CUDA_TRY(cudaGetLastError());
   count_launch(2);
   return BDDA_OK;

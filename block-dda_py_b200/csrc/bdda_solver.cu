@@ -123,8 +123,12 @@ __global__ void cholqr_step_kernel(SmallPtrs s, int L, int first, double shift_c
     }
     __syncthreads();
   }
-  chol_upper(g, L, &bad);
-  tri_upper_inv(g, L, x);
+  if (L <= kElimMax) {
+    elim_chol_inv(g, L, x, &bad);
+  } else {
+    chol_upper(g, L, &bad);
+    tri_upper_inv(g, L, x);
+  }
   block_copy(s.rinv, x, L * L);
   // tau <- R tau
   if (first) {
@@ -145,16 +149,22 @@ __global__ void cocg_alpha_kernel(SmallPtrs s, int L, SolverState* st) {
   extern __shared__ double2 sm[];
   double2* a = sm;
   double2* b = sm + L * L;
-  double2* c = sm + 2 * L * L;
+  double2* c = sm + 2 * L * L + L;
   __shared__ int piv[kMaxL];
   __shared__ int bad;
   if (threadIdx.x == 0) bad = 0;
-  block_copy(a, s.g2, L * L);
-  block_copy(b, s.qq, L * L);
-  __syncthreads();
-  lu_factor(a, L, piv, &bad);
-  if (!bad) lu_solve(a, piv, L, b, L);
   block_copy(c, s.xi, L * L);
+  if (L <= kElimMax) {
+    elim_solve(a, s.g2, s.qq, L, piv, &bad, s.tmp);
+    __syncthreads();
+    block_copy(b, s.tmp, L * L);
+  } else {
+    block_copy(a, s.g2, L * L);
+    block_copy(b, s.qq, L * L);
+    __syncthreads();
+    lu_factor(a, L, piv, &bad);
+    if (!bad) lu_solve(a, piv, L, b, L);
+  }
   __syncthreads();
   small_matmul<false>(b, c, a, L);
   for (int e = threadIdx.x; e < L * L; e += blockDim.x) {
@@ -202,7 +212,7 @@ __global__ void cocg_beta_kernel(SmallPtrs s, int L, SolverState* st) {
   extern __shared__ double2 sm[];
   double2* a = sm;
   double2* b = sm + L * L;
-  double2* c = sm + 2 * L * L;
+  double2* c = sm + 2 * L * L + L;
   __shared__ int piv[kMaxL];
   __shared__ int bad;
   if (threadIdx.x == 0) bad = 0;
@@ -211,11 +221,17 @@ __global__ void cocg_beta_kernel(SmallPtrs s, int L, SolverState* st) {
   block_copy(c, s.g2, L * L);
   __syncthreads();
   small_matmul<true>(b, c, s.tmp, L);   // tau^T (Qn^T Qn)
-  block_copy(b, s.tmp, L * L);
+  if (L <= kElimMax) {
+    __syncthreads();
+    elim_solve(a, s.qq, s.tmp, L, piv, &bad, s.beta);
+  } else {
+    block_copy(b, s.tmp, L * L);
+    __syncthreads();
+    lu_factor(a, L, piv, &bad);
+    if (!bad) lu_solve(a, piv, L, b, L);
+    block_copy(s.beta, b, L * L);
+  }
   __syncthreads();
-  lu_factor(a, L, piv, &bad);
-  if (!bad) lu_solve(a, piv, L, b, L);
-  block_copy(s.beta, b, L * L);
   block_copy(s.qq, c, L * L);
   __syncthreads();
   if (threadIdx.x == 0 && bad == 1) atomicExch(&st->bad, 1);
@@ -735,7 +751,7 @@ static int dda_epilogue(const DdaPhys& ph, const T* X, double2* Xout, bool conve
   BDDA_CUDA_TRY(cudaGetLastError());
   count_launch();
   if (converged) {
-    observables_finalize_kernel<<<(L + 63) / 64, 64, 0, st>>>(ph.partial, kDdaObsBlocks, L, ph.k, ph.absorbing,
+    observables_finalize_kernel<<<L, 256, 0, st>>>(ph.partial, kDdaObsBlocks, L, ph.k, ph.absorbing,
                                                                ph.obs);
     BDDA_CUDA_TRY(cudaGetLastError());
     count_launch();
@@ -772,8 +788,8 @@ static int run_solver(int solver, const bdda_plan* p, int L, int n_occ, const vo
   c.st = reinterpret_cast<SolverState*>(w + o.state);
   c.hist_dev = reinterpret_cast<double*>(w + o.hist);
   c.stream = st;
-  c.sm2 = (size_t)2 * L * L * sizeof(double2);
-  c.sm3 = (size_t)3 * L * L * sizeof(double2);
+  c.sm2 = (size_t)small_elems(L, 2) * sizeof(double2);
+  c.sm3 = (size_t)small_elems(L, 3) * sizeof(double2);
   TRY(allow_smem(bicg_alpha_kernel, c.sm2));
   TRY(allow_smem(bicg_zeta_beta_kernel, c.sm2));
   TRY(allow_smem(cholqr_step_kernel, c.sm2));
@@ -888,8 +904,8 @@ static void fill_ctx(Ctx<T>& c, const bdda_plan* p, int L, int n_occ, const void
   c.sp = small_ptrs(w + small);
   c.st = reinterpret_cast<SolverState*>(w + state);
   c.stream = st;
-  c.sm2 = (size_t)2 * L * L * sizeof(double2);
-  c.sm3 = (size_t)3 * L * L * sizeof(double2);
+  c.sm2 = (size_t)small_elems(L, 2) * sizeof(double2);
+  c.sm3 = (size_t)small_elems(L, 3) * sizeof(double2);
 }
 
 // Block-BiCGSTAB in complex64 with FP64 reliable updates (residual

@@ -75,21 +75,37 @@ __device__ __forceinline__ void bicg_alpha_body(const SmallPtrs& s, int L, Solve
   __shared__ int piv[kMaxL];
   __shared__ int bad;
   if (threadIdx.x == 0) bad = 0;
-  block_copy(a, s.g2, L * L);
-  block_copy(b, s.g2 + L * L, L * L);
-  __syncthreads();
-  lu_factor(a, L, piv, &bad);
-  if (!bad) lu_solve(a, piv, L, b, L);
-  for (int e = threadIdx.x; e < L * L; e += blockDim.x) {
-    s.lu[e] = a[e];
-    s.alpha[e] = b[e];
-    s.negalpha[e] = make_double2(-b[e].x, -b[e].y);
+  if (L <= kElimMax) {
+    const int pitch = elim_pitch(2 * L);
+    elim_load(sm, pitch, s.g2, s.g2 + L * L, L, 1.0);
+    __syncthreads();
+    elim_factor(sm, pitch, L, L, piv, &bad);
+    elim_back(sm, pitch, L, L, piv);
+    for (int e = threadIdx.x; e < L * L; e += blockDim.x) {
+      const int i = e / L, j = e - i * L;
+      const double2 v = sm[piv[i] * pitch + L + j];
+      s.lu[e] = sm[i * pitch + j];
+      s.alpha[e] = v;
+      s.negalpha[e] = make_double2(-v.x, -v.y);
+      if (!zfinite(v)) atomicCAS(&st->bad, 0, 2);
+    }
+  } else {
+    block_copy(a, s.g2, L * L);
+    block_copy(b, s.g2 + L * L, L * L);
+    __syncthreads();
+    lu_factor(a, L, piv, &bad);
+    if (!bad) lu_solve(a, piv, L, b, L);
+    for (int e = threadIdx.x; e < L * L; e += blockDim.x) {
+      s.lu[e] = a[e];
+      s.alpha[e] = b[e];
+      s.negalpha[e] = make_double2(-b[e].x, -b[e].y);
+    }
+    flag_nonfinite(b, L * L, st);
   }
   for (int e = threadIdx.x; e < L; e += blockDim.x) s.piv[e] = piv[e];
   __syncthreads();
   if (threadIdx.x == 0 && bad == 1) atomicExch(&st->bad, 1);
   if (threadIdx.x == 0 && bad == 2) atomicCAS(&st->bad, 0, 2);
-  flag_nonfinite(b, L * L, st);
 }
 
 // BiCGSTAB: zeta = tr(Z^H T) / tr(Z^H Z); beta = RV^-1 (-R0^H Z)   (bl_krylov.py:173,184)
@@ -101,14 +117,24 @@ __device__ __forceinline__ void bicg_zeta_beta_body(const SmallPtrs& s, int L, c
   __shared__ double tot[3];
   __shared__ int singular;
   if (threadIdx.x == 0) singular = (st->bad == 1);
+  // the partials of the dots, all loaded at once, then added in order (the
+  // loads one after another were half of this kernel's time)
+  __shared__ double part[3 * kRedBlocks];
+  for (int e = threadIdx.x; e < 3 * nblk; e += blockDim.x) part[e] = dot_partial[e];
+  const int pitch = elim_pitch(2 * L);
+  if (L <= kElimMax) {
+    elim_load(sm, pitch, s.lu, s.g2, L, -1.0);
+  } else {
+    block_copy(a, s.lu, L * L);
+    for (int e = threadIdx.x; e < L * L; e += blockDim.x) b[e] = make_double2(-s.g2[e].x, -s.g2[e].y);
+  }
+  for (int e = threadIdx.x; e < L; e += blockDim.x) piv[e] = s.piv[e];
+  __syncthreads();
   if (threadIdx.x < 3) {
     double acc = 0.0;
-    for (int k = 0; k < nblk; ++k) acc += dot_partial[k * 3 + threadIdx.x];
+    for (int k = 0; k < nblk; ++k) acc += part[k * 3 + threadIdx.x];
     tot[threadIdx.x] = acc;
   }
-  block_copy(a, s.lu, L * L);
-  for (int e = threadIdx.x; e < L * L; e += blockDim.x) b[e] = make_double2(-s.g2[e].x, -s.g2[e].y);
-  for (int e = threadIdx.x; e < L; e += blockDim.x) piv[e] = s.piv[e];
   __syncthreads();
   if (threadIdx.x == 0) {
     const double2 z = make_double2(tot[0] / tot[2], tot[1] / tot[2]);
@@ -117,6 +143,16 @@ __device__ __forceinline__ void bicg_zeta_beta_body(const SmallPtrs& s, int L, c
     if (!zfinite(z)) atomicCAS(&st->bad, 0, 2);
   }
   __syncthreads();
+  if (L <= kElimMax) {
+    if (singular) return;   // the solve stops at this iteration's test
+    elim_replay(sm, pitch, L, L, piv);
+    elim_back(sm, pitch, L, L, piv);
+    for (int e = threadIdx.x; e < L * L; e += blockDim.x) {
+      const int i = e / L, j = e - i * L;
+      s.beta[e] = sm[piv[i] * pitch + L + j];
+    }
+    return;
+  }
   if (!singular) lu_solve(a, piv, L, b, L);
   block_copy(s.beta, b, L * L);
 }
