@@ -20,8 +20,17 @@
 // M^-1 (B - A X) after every 10-fold drop (bdda_tune_mixed) and before stopping, warm
 // restarts while the true residual is above tol).
 //
-// The pencil passes use the generic run-time-radix kernel body (problems
-// have different radix sequences); the Gram, update and dot kernels use the
+// A problem whose axes have two-register-stage kernels (every even 7-smooth
+// length up to 540, X up to 320; complex128 axes that keep their specialised
+// kernels do not) runs its five pencil passes as launches of those, skipped on
+// the device while its flag is clear; the problems' chains run side by side on
+// up to kSides streams.  The products of the other problems share launches of
+// the generic run-time-radix kernel body (problems have different radix
+// sequences), which all of them did before.  39 iterations, 32 problems of
+// 8^3 cells and 8 columns: 32.3 -> 22.3 ms; 256 of 14^3: 703 -> 325; 16 of 18^3
+// and 16 columns: 147 -> 72; one of 12^3: 9.5 -> 4.8; mixed form 45 -> 39, 674 ->
+// 394, 163 -> 109, 10.2 -> 6.4.  No size measured is better off sharing.
+// The Gram, update and dot kernels use the
 // L-specialised bodies, so L is one of 8, 16, 32, 64.
 #include <algorithm>
 #include <climits>
@@ -44,6 +53,7 @@ constexpr int kClsBlas = 5;
 constexpr int kCheckEvery = 4;    // iterations between host reads of the active count
 constexpr int kRowsPerBlasItem = 512;
 constexpr size_t kPencilBudget = 80 * 1024;
+constexpr int kSides = 8;
 
 // ---- device work list -------------------------------------------------------
 struct ListDev {
@@ -589,6 +599,17 @@ struct Engine {
   int gram_grid[2] = {1, 1}, upd_grid = 1, dots_grid = 1, elem_grid = 1;
   size_t gram_smem[2] = {0, 0}, upd_smem = 0;
   unsigned long long launches = 0;
+  // problems with launches of their own: host arguments of a product site, [5][nprob] as on the device
+  struct Chain {
+    int p;
+    LineLaunchFn fn[5];
+    int64_t P0[5];
+  };
+  std::vector<Chain> chains;
+  bool shared = true;               // some problem's passes are in the work list
+  cudaStream_t side[kSides - 1];    // beside st (nside of them)
+  cudaEvent_t fork = nullptr, join[kSides - 1];
+  int nside = 0;
 
   void count(int n = 1) {
     launches += (unsigned long long)n;
@@ -669,14 +690,36 @@ struct Engine {
     if (lt[q] == 4) return pass_lt<KIND, 4>(args, q);
     return pass_lt<KIND, 2>(args, q);
   }
-  // site: 5 x nprob PassArgs, pass-major
-  int mvp(const PassArgs* site) {
+  // site, host: 5 x nprob PassArgs, pass-major; flags: of the listed problems
+  int mvp(const PassArgs* site, const PassArgs* host, const int* flags) {
     const size_t n = (size_t)nprob;
-    BTRY(pass<K_FWD>(site, 0));
-    BTRY(pass<K_FWD>(site + n, 1));
-    BTRY(pass<K_CONV>(site + 2 * n, 2));
-    BTRY(pass<K_INV>(site + 3 * n, 3));
-    BTRY(pass<K_INV>(site + 4 * n, 4));
+    if (nside) {
+      BDDA_CUDA_TRY(cudaEventRecord(fork, st));
+      for (int i = 0; i < nside; ++i) BDDA_CUDA_TRY(cudaStreamWaitEvent(side[i], fork, 0));
+    }
+    // st takes a share of the chains only when it has no shared passes to run
+    const int lanes = nside + (shared ? 0 : 1);
+    for (size_t c = 0; c < chains.size(); ++c) {
+      const Chain& ch = chains[c];
+      const int lane = lanes ? (int)(c % lanes) : nside;
+      for (int q = 0; q < 5; ++q) {
+        PassArgs a = host[q * n + ch.p];
+        a.live = flags + ch.p;
+        BTRY(ch.fn[q](a, ch.P0[q], lane < nside ? side[lane] : st));
+        ++launches;   // counted globally by the launcher
+      }
+    }
+    if (shared) {
+      BTRY(pass<K_FWD>(site, 0));
+      BTRY(pass<K_FWD>(site + n, 1));
+      BTRY(pass<K_CONV>(site + 2 * n, 2));
+      BTRY(pass<K_INV>(site + 3 * n, 3));
+      BTRY(pass<K_INV>(site + 4 * n, 4));
+    }
+    for (int i = 0; i < nside; ++i) {
+      BDDA_CUDA_TRY(cudaEventRecord(join[i], side[i]));
+      BDDA_CUDA_TRY(cudaStreamWaitEvent(st, join[i], 0));
+    }
     return BDDA_OK;
   }
 
@@ -764,6 +807,32 @@ __global__ void copy_int_kernel(int* dst, const int* src, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) dst[i] = src[i];
 }
+
+// Streams beside the solve's own, with the events that fork to and join them.
+struct Sides {
+  cudaStream_t st[kSides - 1];
+  cudaEvent_t fork = nullptr, join[kSides - 1];
+  int n = 0;
+  int open(int want) {
+    BDDA_CUDA_TRY(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    for (; n < want; ++n) {
+      BDDA_CUDA_TRY(cudaEventCreateWithFlags(&join[n], cudaEventDisableTiming));
+      if (cudaStreamCreateWithFlags(&st[n], cudaStreamNonBlocking) != cudaSuccess) {
+        cudaEventDestroy(join[n]);
+        return BDDA_CUDA_ERROR;
+      }
+    }
+    return BDDA_OK;
+  }
+  ~Sides() {
+    for (int i = 0; i < n; ++i) {
+      cudaStreamSynchronize(st[i]);   // joined already, unless a launch failed in between
+      cudaStreamDestroy(st[i]);
+      cudaEventDestroy(join[i]);
+    }
+    if (fork) cudaEventDestroy(fork);
+  }
+};
 
 // One batched solve; T is the precision of the Krylov vectors (complex128 in
 // the mixed form, whose products run in complex64).
@@ -896,10 +965,23 @@ int batch_run(const bdda_batch_problem* pr, int nprob, int mode, int L, double t
                                static_cast<const double2*>(jpreT), static_cast<double2*>(dst),
                                reinterpret_cast<double2*>(w + q.field), pa, P0);
       const int list = f32 && mixed ? 1 : 0;
+      bool chain = false;
+      {
+        LineLaunchFn fn[5];
+        chain = mvp_line(f32 ? 1 : 0, pa, fn);
+        auto add = [&](auto& eng) {
+          typename std::remove_reference<decltype(eng)>::type::Chain ch;
+          ch.p = i;
+          for (int ps = 0; ps < 5; ++ps) { ch.fn[ps] = fn[ps]; ch.P0[ps] = P0[ps]; }
+          if (eng.chains.empty() || eng.chains.back().p != i) eng.chains.push_back(ch);
+        };
+        if (chain && f32 && mixed) add(e32);
+        else if (chain) add(e);
+      }
       for (int ps = 0; ps < 5; ++ps) {
         pa[ps].ntile = (L + ltv[ps] - 1) / ltv[ps];
         hmvp[((size_t)site * 5 + ps) * np + i] = pa[ps];
-        hcnt[((size_t)list * kNCls + ps) * np + i] = P0[ps] * pa[ps].P1 * pa[ps].ntile;
+        hcnt[((size_t)list * kNCls + ps) * np + i] = chain ? 0 : P0[ps] * pa[ps].P1 * pa[ps].ntile;
       }
     };
     const bool t32 = std::is_same<T, float2>::value;
@@ -926,6 +1008,35 @@ int batch_run(const bdda_batch_problem* pr, int nprob, int mode, int L, double t
       { ElemArgs& x = E(EL_O2Z); x.n = rows * L; x.a = Z; x.b = w + q.out32; }
     }
   }
+  e.shared = e.chains.size() < np;
+  e32.shared = e32.chains.size() < np;
+  Sides sides;
+  {
+    const int nc = (int)std::max(e.chains.size(), e32.chains.size());
+    if (nc > 1) BTRY(sides.open(std::min(nc, kSides) - 1));
+    auto give = [&](auto& eng) {
+      eng.nside = std::min(sides.n, (int)eng.chains.size());
+      eng.fork = sides.fork;
+      for (int i = 0; i < sides.n; ++i) { eng.side[i] = sides.st[i]; eng.join[i] = sides.join[i]; }
+    };
+    give(e);
+    give(e32);
+  }
+  // Mixed form: the complex64 passes of a chained problem read P or T and write V
+  // or Z themselves (site 0 and 1, complex128); its conversions are empty.
+  if (mixed)
+    for (const auto& ch : e32.chains) {
+      const size_t i = (size_t)ch.p;
+      for (int site = 0; site < 2; ++site) {
+        for (int ps = 0; ps < 5; ++ps) hmvp[((size_t)site * 5 + ps) * np + i] = hmvp[(size_t)ps * np + i];
+        PassArgs& z0 = hmvp[((size_t)site * 5 + 0) * np + i];
+        PassArgs& z1 = hmvp[((size_t)site * 5 + 4) * np + i];
+        z0.wide = z1.wide = 1;
+        z0.S = z0.src = z1.S = site == 0 ? hupd[(size_t)U_P * np + i].out : hupd[(size_t)U_T * np + i].out;
+        z1.dst = w + lay.p[i].vec[site == 0 ? 4 : 6];
+      }
+      for (int s : {EL_P2S, EL_T2S, EL_O2V, EL_O2Z}) hel[(size_t)s * np + i].n = 0;
+    }
   for (int list = 0; list < 2; ++list)
     for (int c = 0; c < kNCls; ++c) {
       int64_t sum = 0;
@@ -966,13 +1077,14 @@ int batch_run(const bdda_batch_problem* pr, int nprob, int mode, int L, double t
   auto usite = [&](int s) { return dupd + (size_t)s * np; };
   auto esite = [&](int s) { return del + (size_t)s * np; };
   auto msite = [&](int s) { return dmvp + (size_t)s * 5 * np; };
+  auto hsite = [&](int s) { return hmvp.data() + (size_t)s * 5 * np; };
 
   // the product inside the iteration: src -> dst in T, or through complex64 in the mixed form
   auto iter_mvp = [&](int site, int to32, int from32) -> int {
-    if (!mixed) return e.mvp(msite(site));
-    BTRY(e32.elem(esite(to32), E_CONVERT_IN));
-    BTRY(e32.mvp(msite(0)));
-    return e32.elem(esite(from32), E_CONVERT_OUT);
+    if (!mixed) return e.mvp(msite(site), hsite(site), f_active);
+    if (e32.shared) BTRY(e32.elem(esite(to32), E_CONVERT_IN));
+    BTRY(e32.mvp(msite(0), hsite(site), f_active));
+    return e32.shared ? e32.elem(esite(from32), E_CONVERT_OUT) : BDDA_OK;
   };
   // one iteration of block-BiCGSTAB for every listed problem (bl_krylov.py:161-185);
   // the P update of the previous iteration opens it
@@ -996,7 +1108,7 @@ int batch_run(const bdda_batch_problem* pr, int nprob, int mode, int L, double t
     BDDA_CUDA_TRY(cudaGetLastError());
     if (mixed) {   // residual replacement of the flagged problems, complex128 product
       BTRY(e.list_build(f_repl, 0, 0));
-      BTRY(e.mvp(msite(3)));
+      BTRY(e.mvp(msite(3), hsite(3), f_repl));
       BTRY(e.upd(usite(U_REPL)));
       batch_replace_kernel<<<nprob, 256, 0, st>>>(dpd, f_active, ctl + 3, ctl, o);
       e.count();
@@ -1014,7 +1126,7 @@ int batch_run(const bdda_batch_problem* pr, int nprob, int mode, int L, double t
     e.count();
     BDDA_CUDA_TRY(cudaGetLastError());
     if (warm) {   // with the exact product
-      BTRY(e.mvp(msite(2)));
+      BTRY(e.mvp(msite(2), hsite(2), f_active));
       BTRY(e.upd(usite(U_RX0)));
     }
     BTRY(e.upd(usite(U_P0)));
@@ -1082,7 +1194,7 @@ int batch_run(const bdda_batch_problem* pr, int nprob, int mode, int L, double t
         count_launch();
         // the true residual M^-1 (B - A X) with the complex128 product
         BTRY(e.list_build(f_acc, 0, 0));
-        BTRY(e.mvp(msite(2)));
+        BTRY(e.mvp(msite(2), hsite(2), f_acc));
         BTRY(e.upd(usite(U_TRUE)));
         batch_true_residual_kernel<<<nprob, 256, 0, st>>>(dpd, f_acc);
         BDDA_CUDA_TRY(cudaMemsetAsync(o.counters + 1, 0, sizeof(int), st));

@@ -204,6 +204,7 @@ __global__ void __launch_bounds__(LineShape<T, M, KIND>::NT, LineShape<T, M, KIN
   typedef LineShape<T, M, KIND> S;
   constexpr int A = S::A, B = S::B, H = S::H, W = S::W, NT = S::NT;
   const PassArgs& a = la.p;
+  if (a.live && *a.live == 0) return;
   extern __shared__ __align__(128) unsigned char smraw[];
   T* sm = reinterpret_cast<T*>(smraw);              // [M][W]
   T* tw = sm + M * W;                               // [M]
@@ -360,6 +361,7 @@ __global__ void __launch_bounds__(ConvShape<T, M>::NT, ConvShape<T, M>::MINB) co
   typedef ConvShape<T, M> S;
   constexpr int A = S::A, B = S::B, H = S::H, R = S::R, W = 3 * R, NT = S::NT;
   const PassArgs& a = la.p;
+  if (a.live && *a.live == 0) return;
   extern __shared__ __align__(128) unsigned char smraw[];
   T* sm = reinterpret_cast<T*>(smraw);               // [M][W], column comp * R + r
   T* tw = sm + M * W;                                // [M]

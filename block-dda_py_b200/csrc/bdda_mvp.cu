@@ -249,6 +249,14 @@ static LineLaunchFn line_find(int prec, int kind, const PassArgs& a) {
   return nullptr;
 }
 
+bool mvp_line(int prec, const PassArgs a[5], LineLaunchFn fn[5]) {
+  for (int q = 0; q < 5; ++q) {
+    fn[q] = prec == 0 && fixed_long(kPassKind[q], a[q].ax) ? nullptr : line_find(prec, kPassKind[q], a[q]);
+    if (!fn[q]) return false;
+  }
+  return true;
+}
+
 // Generic kernels: variant -1 with the first stage's global loads, -2 with the
 // TMA-filled tile; with no choice made (variant 0) and no specialised kernel
 // for the radix sequence, the TMA-filled one where the pass allows it.

@@ -45,6 +45,7 @@ struct PassArgs {
   double lf, k;
   unsigned int* err;    // bounded waits that gave up (the plan's counter; null: not counted)
   int wide;             // complex64 passes: S (Z gather, Z^-1 epilogue) and the Z^-1 output are complex128
+  const int* live;      // line kernels: the pass does nothing while *live is 0 (null: always run)
 };
 
 // Element m of a complex128 array as complex64 (round to nearest) and back.
@@ -567,6 +568,9 @@ struct LineKernel {
   int M;
   LineLaunchFn fn;
 };
+// Line kernels (bdda_line.cuh) of the five passes whose arguments a holds; false
+// if one of them has none, or keeps its specialised kernel.
+bool mvp_line(int prec, const PassArgs a[5], LineLaunchFn fn[5]);
 typedef const LineKernel* (*LineTableFn)(int* n);
 #define BDDA_LINE_TABLES(F)                                                                            \
   F(0, K_FWD, line_fwd_c128_a) F(0, K_FWD, line_fwd_c128_b) F(0, K_FWD, line_fwd_c128_c)               \
