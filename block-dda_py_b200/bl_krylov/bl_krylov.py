@@ -256,6 +256,8 @@ _SIZE_RATIO = 1.6
 # Lattices of at least this many padded grid points run the one-problem solver
 # (specialised, autotuned kernels; their launch overhead is negligible there).
 _BATCH_MAX_POINTS = 4 << 20
+# Batch workspaces up to this size are left to torch's allocator after the call.
+_BATCH_KEEP_BYTES = 4 << 30
 
 
 def _batch_groups(entries, mode, L, itermax, max_bytes):
@@ -320,16 +322,25 @@ def bl_bicgstab_jacobi_mvp_fft_batch(problems, tol, itermax, precision=None, max
     itermax = int(itermax)
     dev = entries[0]["g"].plan.device
     fixed_bound = max_bytes is not None
-    if not fixed_bound:
-        torch.cuda.empty_cache()
-        free, _ = torch.cuda.mem_get_info(dev)
-        max_bytes = int(0.7 * free)
     lib = _lib.load()
     results = [None] * len(entries)
     hists = [None] * len(entries)
     big = [i for i, e in enumerate(entries) if int(np.prod(e["g"].plan.m)) >= _BATCH_MAX_POINTS]
     small = [i for i in range(len(entries)) if i not in set(big)]
-    groups = [[small[j] for j in g] for g in _batch_groups([entries[i] for i in small], mode, L, itermax, max_bytes)]
+    split = lambda bound: _batch_groups([entries[i] for i in small], mode, L, itermax, bound)
+    if fixed_bound:
+        groups = split(max_bytes)
+    else:
+        # memory that torch's allocator holds counts as free once it is given
+        # back; that (and taking the workspace from the device anew) costs over a
+        # millisecond a call, so only when it decides how the batch is split
+        free, total = torch.cuda.mem_get_info(dev)
+        groups = split(int(0.7 * free))
+        if groups != split(total):
+            torch.cuda.empty_cache()
+            free, total = torch.cuda.mem_get_info(dev)
+            groups = split(int(0.7 * free))
+    groups = [[small[j] for j in g] for g in groups]
     for g in [g for g in groups if len(g) == 1]:
         big.append(g[0])
     groups = [g for g in groups if len(g) > 1]
@@ -363,7 +374,8 @@ def bl_bicgstab_jacobi_mvp_fft_batch(problems, tol, itermax, precision=None, max
         if rc not in (0, 1, 2):
             _lib.check(rc, "bdda_batch_bicgstab")
         del work
-        torch.cuda.empty_cache()
+        if nb > _BATCH_KEEP_BYTES:   # a smaller one stays with torch's allocator for the next call
+            torch.cuda.empty_cache()
         for i, e in enumerate(grp):
             s = int(st[i])
             X = None if s == 2 else (e["X"].cpu().numpy() if e["numpy"] else e["X"])

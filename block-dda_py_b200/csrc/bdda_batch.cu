@@ -11,7 +11,7 @@
 // (problem, item) pairs from that list.  Converged problems drop out of the
 // list, so they cost nothing, and no host decision is needed per iteration:
 // each problem's convergence test runs on the device.  The iteration is
-// captured once as a CUDA graph and replayed; the host reads one counter
+// captured once as a CUDA graph and replayed after the first few; the host reads one counter
 // (problems still iterating) every kCheckEvery replays.
 //
 // Modes: complex128; complex64; and the mixed form of bdda_mixed_solve
@@ -27,15 +27,17 @@
 // up to kSides streams.  The products of the other problems share launches of
 // the generic run-time-radix kernel body (problems have different radix
 // sequences), which all of them did before.  39 iterations, 32 problems of
-// 8^3 cells and 8 columns: 32.3 -> 22.3 ms; 256 of 14^3: 703 -> 325; 16 of 18^3
-// and 16 columns: 147 -> 72; one of 12^3: 9.5 -> 4.8; mixed form 45 -> 39, 674 ->
-// 394, 163 -> 109, 10.2 -> 6.4.  No size measured is better off sharing.
+// 8^3 cells and 8 columns: 32.9 -> 26.2 ms; 256 of 14^3: 703 -> 365; 16 of 18^3
+// and 16 columns: 147 -> 70; one of 12^3: 9.5 -> 4.5; mixed form 45 -> 44, 674 ->
+// 460, 163 -> 101, 10.2 -> 5.8.  No size measured is better off sharing.
 // The Gram, update and dot kernels use the
 // L-specialised bodies, so L is one of 8, 16, 32, 64.
 #include <algorithm>
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <type_traits>
 #include <vector>
 
@@ -51,6 +53,11 @@ constexpr int kMaxBatch = 1024;   // problems per call (one CTA builds the work 
 constexpr int kNCls = 6;          // work-item classes: the 5 pencil passes, then block kernels
 constexpr int kClsBlas = 5;
 constexpr int kCheckEvery = 4;    // iterations between host reads of the active count
+// Iterations before the iteration's graph is built: a launch in the graph saves
+// 2 us an iteration and costs 15 us to build and release, so a batch that ends
+// within as many iterations as pay for it goes without (4 iterations of 8
+// problems of 16,000 cells: 1.5 ms of 8.5).
+constexpr int kDirect = 8;
 constexpr int kRowsPerBlasItem = 512;
 constexpr size_t kPencilBudget = 80 * 1024;
 constexpr int kSides = 8;
@@ -808,16 +815,59 @@ __global__ void copy_int_kernel(int* dst, const int* src, int n) {
   if (i < n) dst[i] = src[i];
 }
 
+// Idle non-blocking streams of each device, handed out to one solve at a time:
+// creating and destroying one costs 130 us, eight of them 1 ms of a 9 ms
+// batch.  At most kSides idle ones are kept per device (for the life of the
+// process: nothing is destroyed after the driver's own teardown has begun).
+class StreamPool {
+ public:
+  static StreamPool& get() {
+    static StreamPool* pool = new StreamPool;
+    return *pool;
+  }
+  cudaStream_t take(int dev) {
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      std::vector<cudaStream_t>& v = idle_[dev];
+      if (!v.empty()) {
+        cudaStream_t s = v.back();
+        v.pop_back();
+        return s;
+      }
+    }
+    cudaStream_t s = nullptr;
+    return cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess ? s : nullptr;
+  }
+  // s has no work left (a stream with an error is not kept)
+  void give(int dev, cudaStream_t s, bool good) {
+    if (good) {
+      std::lock_guard<std::mutex> lk(mu_);
+      std::vector<cudaStream_t>& v = idle_[dev];
+      if (v.size() < (size_t)kSides) {
+        v.push_back(s);
+        return;
+      }
+    }
+    cudaStreamDestroy(s);
+  }
+
+ private:
+  std::mutex mu_;
+  std::map<int, std::vector<cudaStream_t>> idle_;
+};
+
 // Streams beside the solve's own, with the events that fork to and join them.
 struct Sides {
   cudaStream_t st[kSides - 1];
   cudaEvent_t fork = nullptr, join[kSides - 1];
-  int n = 0;
+  int n = 0, dev = 0;
   int open(int want) {
+    BDDA_CUDA_TRY(cudaGetDevice(&dev));
     BDDA_CUDA_TRY(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
     for (; n < want; ++n) {
       BDDA_CUDA_TRY(cudaEventCreateWithFlags(&join[n], cudaEventDisableTiming));
-      if (cudaStreamCreateWithFlags(&st[n], cudaStreamNonBlocking) != cudaSuccess) {
+      st[n] = StreamPool::get().take(dev);
+      if (!st[n]) {
         cudaEventDestroy(join[n]);
         return BDDA_CUDA_ERROR;
       }
@@ -826,8 +876,8 @@ struct Sides {
   }
   ~Sides() {
     for (int i = 0; i < n; ++i) {
-      cudaStreamSynchronize(st[i]);   // joined already, unless a launch failed in between
-      cudaStreamDestroy(st[i]);
+      // joined already, unless a launch failed in between
+      StreamPool::get().give(dev, st[i], cudaStreamSynchronize(st[i]) == cudaSuccess);
       cudaEventDestroy(join[i]);
     }
     if (fork) cudaEventDestroy(fork);
@@ -1153,9 +1203,9 @@ int batch_run(const bdda_batch_problem* pr, int nprob, int mode, int L, double t
     count_launch(-(int)per_iter);   // captured, not run
     return BDDA_OK;
   };
-  // iterate until every listed problem stopped (or maxit iterations)
+  // iterate until every listed problem stopped (or maxit iterations); the graph
+  // is built once kDirect iterations are launched, while they run
   auto run_iterations = [&](int maxit) -> int {
-    BTRY(capture());
     int done = 0;
     while (done < maxit) {
       const int n = std::min(kCheckEvery, maxit - done);
@@ -1168,6 +1218,7 @@ int batch_run(const bdda_batch_problem* pr, int nprob, int mode, int L, double t
         }
       }
       done += n;
+      if (done >= kDirect && done < maxit) BTRY(capture());
       int left = 0;
       BDDA_CUDA_TRY(cudaMemcpyAsync(&left, ctl + 3, sizeof(int), cudaMemcpyDeviceToHost, st));
       BDDA_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1256,11 +1307,13 @@ int bdda_batch_bicgstab(const bdda_batch_problem* problems, int nprob, int mode,
   unsigned char* w = static_cast<unsigned char*>(work);
   cudaStream_t user = static_cast<cudaStream_t>(stream);
   // an own stream, ordered after the caller's: a graph cannot capture the legacy stream
-  cudaStream_t st = nullptr;
+  int dev = 0;
+  BDDA_CUDA_TRY(cudaGetDevice(&dev));
+  cudaStream_t st = StreamPool::get().take(dev);
+  if (!st) return BDDA_CUDA_ERROR;
   cudaEvent_t ev = nullptr;
-  BDDA_CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
   if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
-    cudaStreamDestroy(st);
+    StreamPool::get().give(dev, st, true);
     return BDDA_CUDA_ERROR;
   }
   int rc = BDDA_CUDA_ERROR;
@@ -1273,8 +1326,7 @@ int bdda_batch_bicgstab(const bdda_batch_problem* problems, int nprob, int mode,
   }
   cudaEventRecord(ev, st);
   cudaStreamWaitEvent(user, ev, 0);
-  cudaStreamSynchronize(st);
-  cudaStreamDestroy(st);
+  StreamPool::get().give(dev, st, cudaStreamSynchronize(st) == cudaSuccess);
   cudaEventDestroy(ev);
   return rc;
 }

@@ -542,16 +542,23 @@ static int cocg_core(Ctx<T>& c, bool has_x0, double tol, int itermax, int* iter_
 // the iteration, and keep looping while err >= tol, no breakdown or
 // non-finite value, and iterations remain.  The loop condition is the graph's
 // while-node handle; the counter bounds the loop by itermax whatever happens.
+__device__ __forceinline__ int loop_record(SolverState* st, double* hist) {
+  const int k = st->iter;
+  if (k < kGraphHistCap) hist[k] = st->err;
+  st->iter = k + 1;
+  return k;
+}
 __global__ void loop_check_kernel(SolverState* st, double tol, int itermax, double* hist,
                                   cudaGraphConditionalHandle h) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const int k = st->iter;
+  const int k = loop_record(st, hist);
   const double err = st->err;
-  if (k < kGraphHistCap) hist[k] = err;
-  st->iter = k + 1;
   const bool go = st->bad == 0 && !(err < tol) && k + 1 < itermax;
   cudaGraphSetConditional(h, go ? 1u : 0u);
 }
+
+// The same record of an iteration that the host drives.
+__global__ void loop_record_kernel(SolverState* st, double* hist) { loop_record(st, hist); }
 
 // Non-blocking stream per device for capturing the loop bodies (the caller's
 // stream may be the legacy default stream, which cannot be captured).
@@ -566,69 +573,120 @@ static cudaStream_t capture_stream() {
   return streams[dev];
 }
 
-// Graph-driven loop: one while node whose body is `body(cc, h)` captured on a
-// private stream (cc = c with that stream), then one launch on c.stream and
-// one read-back.  Returns BDDA_OK / BREAKDOWN / NOT_CONVERGED like the
-// host-driven cores; any failure while building the graph returns
-// BDDA_CUDA_ERROR before anything ran (the caller then runs the host loop).
-template <typename T, typename Body>
-static int graph_loop(Ctx<T>& c, double tol, int itermax, int* iter_fin, double* err_fin, double* hist,
-                      Body body) {
-  cudaStream_t cs = capture_stream();
-  if (!cs) return BDDA_CUDA_ERROR;
+// Iterations that the host drives before the loop's graph is built.  Building
+// and releasing it costs 460 us, reading the state back 15 us an iteration: a
+// solve that ends within these is faster without (5 iterations of a 1,100-cell
+// particle with 16 columns: a third of the call), and a longer one pays nothing,
+// because the graph is built while the last of them runs.
+constexpr int kHostIters = 8;
+
+// The loop: step(cc) is an iteration up to its test, next(cc) prepares the
+// following one.  The first kHostIters are driven by the host on c.stream; the
+// others are one while node whose body (step, test, next) is captured on a
+// private stream, one launch on c.stream and one read-back.  Returns BDDA_OK /
+// BREAKDOWN / NOT_CONVERGED like the host-driven cores; if the graph cannot be
+// built the host drives the rest.
+template <typename T, typename Step, typename Next>
+static int graph_loop(Ctx<T>& c, double tol, int itermax, int* iter_fin, double* err_fin, double* hist, Step step,
+                      Next next) {
   cudaGraph_t g = nullptr;
   cudaGraphExec_t ex = nullptr;
-  cudaGraphConditionalHandle h;
-  int status = BDDA_CUDA_ERROR;
-  long long n0 = 0, nbody = 0;
-  do {
-    if (cudaGraphCreate(&g, 0) != cudaSuccess) break;
-    if (cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault) != cudaSuccess) break;
-    cudaGraphNodeParams np = {cudaGraphNodeTypeConditional};
-    np.conditional.handle = h;
-    np.conditional.type = cudaGraphCondTypeWhile;
-    np.conditional.size = 1;
-    cudaGraphNode_t node;
-    if (cudaGraphAddNode(&node, g, nullptr, 0, &np) != cudaSuccess) break;
-    cudaGraph_t bodyg = np.conditional.phGraph_out[0];
-    Ctx<T> cc = c;
-    cc.stream = cs;
-    if (cudaStreamBeginCaptureToGraph(cs, bodyg, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) != cudaSuccess)
+  long long nbody = 0;
+  auto build = [&]() {
+    cudaStream_t cs = capture_stream();
+    if (!cs) return;
+    cudaGraphConditionalHandle h;
+    bool ok = false;
+    do {
+      if (cudaGraphCreate(&g, 0) != cudaSuccess) break;
+      if (cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault) != cudaSuccess) break;
+      cudaGraphNodeParams np = {cudaGraphNodeTypeConditional};
+      np.conditional.handle = h;
+      np.conditional.type = cudaGraphCondTypeWhile;
+      np.conditional.size = 1;
+      cudaGraphNode_t node;
+      if (cudaGraphAddNode(&node, g, nullptr, 0, &np) != cudaSuccess) break;
+      Ctx<T> cc = c;
+      cc.stream = cs;
+      if (cudaStreamBeginCaptureToGraph(cs, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                        cudaStreamCaptureModeRelaxed) != cudaSuccess)
+        break;
+      const long long n0 = bdda_launch_count();
+      int sb = step(cc);
+      if (sb == BDDA_OK) {
+        loop_check_kernel<<<1, 32, 0, cs>>>(cc.st, tol, itermax, cc.hist_dev, h);
+        count_launch();
+        sb = next(cc);
+      }
+      cudaGraph_t captured = nullptr;
+      const cudaError_t ec = cudaStreamEndCapture(cs, &captured);
+      nbody = bdda_launch_count() - n0;
+      count_launch((int)-nbody);   // captured, not run
+      if (sb != BDDA_OK || ec != cudaSuccess) break;
+      ok = cudaGraphInstantiate(&ex, g, 0) == cudaSuccess;
+    } while (false);
+    if (!ok) {
+      cudaGetLastError();
+      if (g) cudaGraphDestroy(g);
+      g = nullptr;
+      ex = nullptr;
+    }
+  };
+  int rc = BDDA_NOT_CONVERGED, k = 0;
+  bool on = false;   // the graph runs the iterations from k
+  while (k < itermax && !on) {
+    rc = step(c);
+    if (rc == BDDA_OK) {
+      loop_record_kernel<<<1, 1, 0, c.stream>>>(c.st, c.hist_dev);
+      count_launch();
+      if (cudaGetLastError() != cudaSuccess) rc = BDDA_CUDA_ERROR;
+    }
+    if (rc == BDDA_OK && k + 1 == kHostIters && k + 1 < itermax) build();
+    double err = INFINITY;
+    int bad = 0;
+    if (rc == BDDA_OK) rc = read_state(c, &err, &bad);
+    if (rc == BDDA_OK && bad == 1) rc = BDDA_BREAKDOWN;
+    if (rc != BDDA_OK) break;
+    if (hist) hist[k] = err;
+    *iter_fin = k++;
+    *err_fin = err;
+    if (bad != 2 && err < tol) break;
+    rc = BDDA_NOT_CONVERGED;
+    if (bad == 2 || k == itermax) break;
+    const int s = next(c);
+    if (s != BDDA_OK) {
+      rc = s;
       break;
-    n0 = bdda_launch_count();
-    const int sb = body(cc, h);
-    cudaGraph_t captured = nullptr;
-    const cudaError_t ec = cudaStreamEndCapture(cs, &captured);
-    nbody = bdda_launch_count() - n0;
-    if (sb != BDDA_OK || ec != cudaSuccess) break;
-    if (cudaGraphInstantiate(&ex, g, 0) != cudaSuccess) break;
-    status = BDDA_OK;
-  } while (false);
-  if (status != BDDA_OK) {
-    cudaGetLastError();
-    if (ex) cudaGraphExecDestroy(ex);
-    if (g) cudaGraphDestroy(g);
-    return BDDA_CUDA_ERROR;
+    }
+    on = ex != nullptr;
   }
-  const cudaError_t el = cudaGraphLaunch(ex, c.stream);
-  SolverState hs;
-  const cudaError_t ec = el == cudaSuccess ? cudaMemcpyAsync(&hs, c.st, sizeof(hs), cudaMemcpyDeviceToHost, c.stream)
-                                           : el;
-  const cudaError_t es = ec == cudaSuccess ? cudaStreamSynchronize(c.stream) : ec;
-  cudaGraphExecDestroy(ex);
-  cudaGraphDestroy(g);
-  if (es != cudaSuccess) return BDDA_CUDA_ERROR;
-  const int ran = hs.iter < 1 ? 1 : (hs.iter > itermax ? itermax : hs.iter);
-  count_launch((int)(nbody * (ran - 1)));   // the body was counted once, at capture
-  if (hist) {
-    const int nh = ran < kGraphHistCap ? ran : kGraphHistCap;
-    BDDA_CUDA_TRY(cudaMemcpy(hist, c.hist_dev, nh * sizeof(double), cudaMemcpyDeviceToHost));
+  if (on) {
+    SolverState hs;
+    cudaError_t e = cudaGraphLaunch(ex, c.stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&hs, c.st, sizeof(hs), cudaMemcpyDeviceToHost, c.stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
+    if (e == cudaSuccess) {
+      const int ran = hs.iter < k + 1 ? k + 1 : (hs.iter > itermax ? itermax : hs.iter);
+      count_launch((int)(nbody * (ran - k)));
+      const int nh = std::min(ran, kGraphHistCap);
+      if (hist && nh > k)
+        e = cudaMemcpy(hist + k, c.hist_dev + k, (nh - k) * sizeof(double), cudaMemcpyDeviceToHost);
+      if (hs.bad == 1) rc = BDDA_BREAKDOWN;
+      else {
+        *iter_fin = ran - 1;
+        *err_fin = hs.err;
+        rc = hs.bad != 2 && hs.err < tol ? BDDA_OK : BDDA_NOT_CONVERGED;
+      }
+    }
+    if (e != cudaSuccess) rc = BDDA_CUDA_ERROR;
   }
-  if (hs.bad == 1) return BDDA_BREAKDOWN;
-  *iter_fin = ran - 1;
-  *err_fin = hs.err;
-  if (hs.bad == 2) return BDDA_NOT_CONVERGED;
-  return hs.err < tol ? BDDA_OK : BDDA_NOT_CONVERGED;
+  if (ex) cudaGraphExecDestroy(ex);
+  if (g) cudaGraphDestroy(g);
+  if (rc == BDDA_BREAKDOWN) {
+    *iter_fin = 0;
+    *err_fin = INFINITY;
+  }
+  return rc;
 }
 
 // Block-BiCGSTAB with the graph-driven loop (plain forms, no complex64 products
@@ -652,7 +710,7 @@ static int bicgstab_graph(Ctx<T>& c, bool has_x0, double tol, int itermax, int* 
   TRY(upd<T>(c, R0, R, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, false));
   *iter_fin = 0;
   *err_fin = INFINITY;
-  return graph_loop<T>(c, tol, itermax, iter_fin, err_fin, hist, [&](Ctx<T>& cc, cudaGraphConditionalHandle h) -> int {
+  auto step = [&](Ctx<T>& cc) -> int {
     TRY(mvp<T>(cc, P, V));
     TRY(gram2<T>(cc, true, R0, V, R, cc.sp.g2));
     bicg_alpha_kernel<<<1, 256, cc.sm2, cc.stream>>>(cc.sp, L, cc.st);
@@ -668,11 +726,13 @@ static int bicgstab_graph(Ctx<T>& c, bool has_x0, double tol, int itermax, int* 
     TRY(upd<T>(cc, X, X, nullptr, Tt, &cc.st->zeta, P, nullptr, nullptr, cc.sp.alpha, false));
     TRY(upd<T>(cc, R, Tt, nullptr, Z, &cc.st->negzeta, nullptr, nullptr, nullptr, nullptr, true));
     norm_kernel<<<1, 256, 0, cc.stream>>>(reinterpret_cast<double*>(cc.partial), kRedBlocks, cc.st, 0);
-    loop_check_kernel<<<1, 32, 0, cc.stream>>>(cc.st, tol, itermax, cc.hist_dev, h);
-    count_launch(2);
-    TRY(upd<T>(cc, P, R, nullptr, nullptr, nullptr, P, V, &cc.st->negzeta, cc.sp.beta, false));
+    count_launch();
     return cudaGetLastError() == cudaSuccess ? BDDA_OK : BDDA_CUDA_ERROR;
-  });
+  };
+  auto next = [&](Ctx<T>& cc) -> int {
+    return upd<T>(cc, P, R, nullptr, nullptr, nullptr, P, V, &cc.st->negzeta, cc.sp.beta, false);
+  };
+  return graph_loop<T>(c, tol, itermax, iter_fin, err_fin, hist, step, next);
 }
 
 // Block-COCG-rq with the graph-driven loop.  The host loop swaps the roles of
@@ -703,7 +763,7 @@ static int cocg_graph(Ctx<T>& c, bool has_x0, double tol, int itermax, int* iter
   TRY(gram2<T>(c, false, Q, Q, nullptr, c.sp.qq));
   *iter_fin = 0;
   *err_fin = INFINITY;
-  return graph_loop<T>(c, tol, itermax, iter_fin, err_fin, hist, [&](Ctx<T>& cc, cudaGraphConditionalHandle h) -> int {
+  auto step = [&](Ctx<T>& cc) -> int {
     TRY(mvp<T>(cc, S, AS));
     TRY(gram2<T>(cc, false, S, AS, nullptr, cc.sp.g2));
     cocg_alpha_kernel<<<1, 256, cc.sm3, cc.stream>>>(cc.sp, L, cc.st);
@@ -713,8 +773,10 @@ static int cocg_graph(Ctx<T>& c, bool has_x0, double tol, int itermax, int* iter
     T* qn = nullptr;
     TRY(cholqr3<T>(cc, W, Q2, Q3, &qn));   // Qnew in Q2, tau in sp.tau
     cocg_xi_kernel<<<1, 256, cc.sm3, cc.stream>>>(cc.sp, L, cc.st, 0);
-    loop_check_kernel<<<1, 32, 0, cc.stream>>>(cc.st, tol, itermax, cc.hist_dev, h);
-    count_launch(2);
+    count_launch();
+    return cudaGetLastError() == cudaSuccess ? BDDA_OK : BDDA_CUDA_ERROR;
+  };
+  auto next = [&](Ctx<T>& cc) -> int {
     TRY(gram2<T>(cc, false, Q2, Q2, nullptr, cc.sp.g2));
     cocg_beta_kernel<<<1, 256, cc.sm3, cc.stream>>>(cc.sp, L, cc.st);
     count_launch();
@@ -722,7 +784,8 @@ static int cocg_graph(Ctx<T>& c, bool has_x0, double tol, int itermax, int* iter
     if (cudaMemcpyAsync(Q, Q2, (size_t)cc.n * L * sizeof(T), cudaMemcpyDeviceToDevice, cc.stream) != cudaSuccess)
       return BDDA_CUDA_ERROR;
     return cudaGetLastError() == cudaSuccess ? BDDA_OK : BDDA_CUDA_ERROR;
-  });
+  };
+  return graph_loop<T>(c, tol, itermax, iter_fin, err_fin, hist, step, next);
 }
 
 // The host-driven loops are used when the graph-driven one is off
