@@ -196,9 +196,9 @@ __device__ __forceinline__ float2 line_fma(float2 a, float2 b, float2 c) {
 template <typename T> __device__ __forceinline__ T czero() { return mkc<T>(0, 0); }
 
 // ---- forward / inverse pass --------------------------------------------------------
-// FULL: the forward pass of a pencil whose M rows all hold data (the Green's
-// tensor): the even half transforms x[q] + x[q + H], the odd one their
-// difference.
+// FULL: the forward pass of a pencil with data in its upper half too, the images
+// of the rows below (the Green's tensor; PassArgs.mirror): the even half
+// transforms x[q] + x[q + H], the odd one their difference.
 template <typename T, int KIND, int M, bool FULL>
 __global__ void __launch_bounds__(LineShape<T, M, KIND>::NT, LineShape<T, M, KIND>::MINB) line_kernel(const __grid_constant__ LineArgs la) {
   typedef LineShape<T, M, KIND> S;
@@ -253,8 +253,14 @@ __global__ void __launch_bounds__(LineShape<T, M, KIND>::NT, LineShape<T, M, KIN
       } else {
 #pragma unroll
         for (int q = 0; q < H; ++q) {
-          const T lo = col ? src[(int64_t)(j + B * q) * a.src_row] : czero<T>();
-          const T hi = col ? src[(int64_t)(j + B * (q + H)) * a.src_row] : czero<T>();
+          // row r, and row r + M / 2, the image of row M / 2 - r
+          const int r = j + B * q, i = M / 2 - r;
+          const T lo = col && r < a.n_in ? src[(int64_t)r * a.src_row] : czero<T>();
+          T hi = col && i < a.n_in ? src[(int64_t)i * a.src_row] : czero<T>();
+          if ((a.mirror >> c) & 1) {
+            hi.x = -hi.x;
+            hi.y = -hi.y;
+          }
           t[q] = cadd(lo, hi);
           x[q] = csub(lo, hi);
         }

@@ -45,6 +45,7 @@ struct PassArgs {
   double lf, k;
   unsigned int* err;    // bounded waits that gave up (the plan's counter; null: not counted)
   int wide;             // complex64 passes: S (Z gather, Z^-1 epilogue) and the Z^-1 output are complex128
+  int mirror;           // line kernels, K_FWD: row M - i is row i (i < n_in) with the columns of these bits negated
   const int* live;      // line kernels: the pass does nothing while *live is 0 (null: always run)
 };
 
@@ -561,8 +562,7 @@ struct FixedKernel {
   int pair;            // 1: column-pair jobs (needs even L and 16-byte aligned fields)
 };
 // Two-register-stage kernels of one axis length (bdda_line.cuh), tables by
-// precision, pass kind (3: a forward pass whose M rows all hold data) and
-// length range.
+// precision, pass kind (3: a forward pass over mirrored rows) and length range.
 typedef int (*LineLaunchFn)(const PassArgs& a, int64_t P0, cudaStream_t st);
 struct LineKernel {
   int M;
