@@ -71,6 +71,24 @@ __device__ __forceinline__ float pow2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
+// Two values at once: the packed FMA of sm_100 does both in one issue slot, with the same rounding.
+typedef unsigned long long pair2;
+__device__ __forceinline__ pair2 pack2(float x, float y) {
+  pair2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(pair2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ pair2 both(float x) { return pack2(x, x); }
+__device__ __forceinline__ pair2 fma2(pair2 a, pair2 b, pair2 c) {
+  pair2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
 // Normal distribution function Phi(z) = erfc(-z / sqrt 2) / 2 without a branch:
 // erfc(a) = 2^q(a) for a = |z| / sqrt 2 <= 6, q a polynomial of degree 12 with
 // q(0) = 0 fitted to log2 erfc (weighted least squares, iterated to the
@@ -78,30 +96,37 @@ __device__ __forceinline__ float pow2(float x) {
 // as 0.5 (1 + erff) is, for 17 instructions instead of about 40 (erff runs
 // both of its branches in most warps; GELU was two thirds of the projection's
 // instructions).
-__device__ __forceinline__ float normal_cdf(float z) {
-  const float a = fminf(fabsf(z) * 0.70710678118654752f, 16.0f);
-  float q = -8.052739808e-09f;
-  q = fmaf(q, a, 2.966770865e-07f);
-  q = fmaf(q, a, -4.839806024e-06f);
-  q = fmaf(q, a, 4.601462206e-05f);
-  q = fmaf(q, a, -2.808824938e-04f);
-  q = fmaf(q, a, 1.121692010e-03f);
-  q = fmaf(q, a, -2.623979701e-03f);
-  q = fmaf(q, a, 3.509852104e-04f);
-  q = fmaf(q, a, 2.760771848e-02f);
-  q = fmaf(q, a, -1.482808441e-01f);
-  q = fmaf(q, a, -9.184457064e-01f);
-  q = fmaf(q, a, -1.627907157e+00f);
-  const float e = 0.5f * pow2(q * a);
-  return z < 0.f ? e : 1.0f - e;
+__device__ __forceinline__ float2 normal_cdf(float2 z) {
+  const float ax = fminf(fabsf(z.x) * 0.70710678118654752f, 16.0f);
+  const float ay = fminf(fabsf(z.y) * 0.70710678118654752f, 16.0f);
+  const pair2 a = pack2(ax, ay);
+  pair2 q = both(-8.052739808e-09f);
+  q = fma2(q, a, both(2.966770865e-07f));
+  q = fma2(q, a, both(-4.839806024e-06f));
+  q = fma2(q, a, both(4.601462206e-05f));
+  q = fma2(q, a, both(-2.808824938e-04f));
+  q = fma2(q, a, both(1.121692010e-03f));
+  q = fma2(q, a, both(-2.623979701e-03f));
+  q = fma2(q, a, both(3.509852104e-04f));
+  q = fma2(q, a, both(2.760771848e-02f));
+  q = fma2(q, a, both(-1.482808441e-01f));
+  q = fma2(q, a, both(-9.184457064e-01f));
+  q = fma2(q, a, both(-1.627907157e+00f));
+  const float2 v = unpack2(q);
+  const float ex = 0.5f * pow2(v.x * ax), ey = 0.5f * pow2(v.y * ay);
+  return make_float2(z.x < 0.f ? ex : 1.0f - ex, z.y < 0.f ? ey : 1.0f - ey);
 }
 // its derivative exp(-z^2 / 2) / sqrt(2 pi)
 __device__ __forceinline__ float normal_pdf(float z) {
   return 0.39894228040143268f * pow2(-0.72134752044448170f * z * z);
 }
-__device__ __forceinline__ float gelu(float z) { return z * normal_cdf(z); }
-__device__ __forceinline__ float gelu_grad(float z) {
-  return fmaf(z, normal_pdf(z), normal_cdf(z));
+__device__ __forceinline__ float2 gelu(float2 z) {
+  const float2 c = normal_cdf(z);
+  return make_float2(z.x * c.x, z.y * c.y);
+}
+__device__ __forceinline__ float2 gelu_grad(float2 z) {
+  const float2 c = normal_cdf(z);
+  return make_float2(fmaf(z.x, normal_pdf(z.x), c.x), fmaf(z.y, normal_pdf(z.y), c.y));
 }
 
 // ---- tensor-core pointwise layers --------------------------------------------------------------
@@ -384,7 +409,7 @@ __global__ void __launch_bounds__(256, 3) layer_fwd_kernel(const float* v, const
           if (m >= m1) continue;
           const float z0 = acc[ns][2 * hr] + bs[c], z1 = acc[ns][2 * hr + 1] + bs[c + 1];
           if (z) *reinterpret_cast<float2*>(z + m * kW + c) = make_float2(z0, z1);
-          *reinterpret_cast<float2*>(y + m * kW + c) = act ? make_float2(gelu(z0), gelu(z1)) : make_float2(z0, z1);
+          *reinterpret_cast<float2*>(y + m * kW + c) = act ? gelu(make_float2(z0, z1)) : make_float2(z0, z1);
         }
     }
   }
@@ -437,13 +462,14 @@ __global__ void __launch_bounds__(256, 3) proj_fwd_kernel(const float* v, const 
         const int64_t m = m0 + g + 8 * hr;
         if (zq && m < M) *reinterpret_cast<float2*>(zq + m * kProj + c) = make_float2(acc[ns][2 * hr], acc[ns][2 * hr + 1]);
       }
+      const float2 h2[2] = {gelu(make_float2(acc[ns][0], acc[ns][1])), gelu(make_float2(acc[ns][2], acc[ns][3]))};
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
         const float4 wa = *reinterpret_cast<const float4*>(w2 + (c + q) * 8);
         const float2 wb = *reinterpret_cast<const float2*>(w2 + (c + q) * 8 + 4);
 #pragma unroll
         for (int hr = 0; hr < 2; ++hr) {
-          const float h = gelu(acc[ns][2 * hr + q]);
+          const float h = q ? h2[hr].y : h2[hr].x;
           out[hr][0] = fmaf(h, wa.x, out[hr][0]); out[hr][1] = fmaf(h, wa.y, out[hr][1]);
           out[hr][2] = fmaf(h, wa.z, out[hr][2]); out[hr][3] = fmaf(h, wa.w, out[hr][3]);
           out[hr][4] = fmaf(h, wb.x, out[hr][4]); out[hr][5] = fmaf(h, wb.y, out[hr][5]);
@@ -489,22 +515,18 @@ __global__ void __launch_bounds__(32 * kProjWarps, 3) proj_bwd_kernel(const floa
   float* vt = tiles + warp * TILE;
   float* gt = vt + 16 * kPvS;
   float* yt = gt + 16 * kPgS;
-  float w2[2][kCout], b1[2] = {0.f, 0.f}, b2 = 0.f;
+  pair2 w2[kCout], aq2[kCout];   // rows lane, lane + 32 of Q2 and of its gradient
+  float b1[2] = {0.f, 0.f}, b2 = 0.f;
 #pragma unroll
-  for (int q = 0; q < 2; ++q)
-#pragma unroll
-    for (int o = 0; o < kCout; ++o) w2[q][o] = Q2[(lane + 32 * q) * kCout + o];
-  float aq1[2][kProj / 8][4], aq2[2][kCout];   // aq2: rows lane, lane + 32 of Q2's gradient
+  for (int o = 0; o < kCout; ++o) {
+    w2[o] = pack2(Q2[lane * kCout + o], Q2[(lane + 32) * kCout + o]);
+    aq2[o] = both(0.f);
+  }
+  float aq1[2][kProj / 8][4];
 #pragma unroll
   for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-    for (int ns = 0; ns < kProj / 8; ++ns)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) aq1[mt][ns][q] = 0.f;
-#pragma unroll
-  for (int q = 0; q < 2; ++q)
-#pragma unroll
-    for (int o = 0; o < kCout; ++o) aq2[q][o] = 0.f;
+    for (int ns = 0; ns < kProj / 8; ++ns) aq1[mt][ns][0] = aq1[mt][ns][1] = aq1[mt][ns][2] = aq1[mt][ns][3] = 0.f;
   const int64_t ntile = (M + 15) / 16;
   for (int64_t tile = blockIdx.x * (int64_t)kProjWarps + warp; tile < ntile; tile += (int64_t)gridDim.x * kProjWarps) {
     const int64_t m0 = tile * 16;
@@ -517,27 +539,25 @@ __global__ void __launch_bounds__(32 * kProjWarps, 3) proj_bwd_kernel(const floa
       yt[e] = r < nr && o < kCout ? gy[(m0 + r) * kCout + o] : 0.f;
     }
     __syncwarp();
-#pragma unroll 4
+#pragma unroll 8
     for (int r = 0; r < 16; ++r) {
-      float y6[kCout];
+      pair2 y6[kCout], gh = both(0.f);
 #pragma unroll
-      for (int o = 0; o < kCout; ++o) y6[o] = yt[r * kPyS + o];
+      for (int o = 0; o < kCout; ++o) y6[o] = both(yt[r * kPyS + o]);
+      const float* zr = zq + (m0 + min(r, nr - 1)) * kProj + lane;   // rows past the end: gy is zero
+      const float2 zz = make_float2(zr[0], zr[32]);
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        float gz = 0.f;
-        if (r < nr) {
-          const float zz = zq[(m0 + r) * kProj + lane + 32 * q];
-          float gh = 0.f;
+      for (int o = 0; o < kCout; ++o) gh = fma2(y6[o], w2[o], gh);
+      const float2 cdf = normal_cdf(zz), gy2 = unpack2(gh);
+      const pair2 h = pack2(zz.x * cdf.x, zz.y * cdf.y);
+      const float gx = gy2.x * fmaf(zz.x, normal_pdf(zz.x), cdf.x);
+      const float gw = gy2.y * fmaf(zz.y, normal_pdf(zz.y), cdf.y);
 #pragma unroll
-          for (int o = 0; o < kCout; ++o) gh = fmaf(y6[o], w2[q][o], gh);
-          const float cdf = normal_cdf(zz), h = zz * cdf;
-          gz = gh * fmaf(zz, normal_pdf(zz), cdf);
-#pragma unroll
-          for (int o = 0; o < kCout; ++o) aq2[q][o] = fmaf(h, y6[o], aq2[q][o]);
-        }
-        gt[r * kPgS + lane + 32 * q] = gz;
-        b1[q] += gz;
-      }
+      for (int o = 0; o < kCout; ++o) aq2[o] = fma2(h, y6[o], aq2[o]);
+      gt[r * kPgS + lane] = gx;
+      gt[r * kPgS + lane + 32] = gw;
+      b1[0] += gx;
+      b1[1] += gw;
       if (lane < kCout) b2 += yt[r * kPyS + lane];
     }
     vr.put<kPvS>(vt, lane);
@@ -571,9 +591,11 @@ __global__ void __launch_bounds__(32 * kProjWarps, 3) proj_bwd_kernel(const floa
       for (int q = 0; q < 4; ++q)
         atomicAdd(&rq1[(mt * 16 + g + 8 * (q >> 1)) * kProj + ns * 8 + 2 * t + (q & 1)], aq1[mt][ns][q]);
 #pragma unroll
-  for (int q = 0; q < 2; ++q)
-#pragma unroll
-    for (int o = 0; o < kCout; ++o) atomicAdd(&rq2[(lane + 32 * q) * kCout + o], aq2[q][o]);
+  for (int o = 0; o < kCout; ++o) {
+    const float2 v = unpack2(aq2[o]);
+    atomicAdd(&rq2[lane * kCout + o], v.x);
+    atomicAdd(&rq2[(lane + 32) * kCout + o], v.y);
+  }
   __syncthreads();
   for (int e = threadIdx.x; e < kW * kProj; e += blockDim.x) atomicAdd(&gQ1[e], rq1[e]);
   for (int e = threadIdx.x; e < kProj; e += blockDim.x) atomicAdd(&gq1[e], rb1[e]);
@@ -649,8 +671,9 @@ __global__ void __launch_bounds__(32 * kLayerWarps, 4) layer_bwd_kernel(const fl
           float a = acc[ns][2 * hr], b = acc[ns][2 * hr + 1];
           if (zprev) {
             const float2 zz = *reinterpret_cast<const float2*>(zprev + m * kW + c);
-            a *= gelu_grad(zz.x);
-            b *= gelu_grad(zz.y);
+            const float2 dz = gelu_grad(zz);
+            a *= dz.x;
+            b *= dz.y;
           }
           *reinterpret_cast<float2*>(gout + m * kW + c) = make_float2(a, b);
         }
