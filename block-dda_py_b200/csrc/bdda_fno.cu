@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(256, 3) layer_fwd_kernel(const float* v, const
 }
 
 // ---- projection: y = gelu(v Q1 + q1) Q2 + q2; the hidden pre-activation is kept for training ----
-__global__ void __launch_bounds__(256, 3) proj_fwd_kernel(const float* v, const float* Q1, const float* q1,
+__global__ void __launch_bounds__(256, 2) proj_fwd_kernel(const float* v, const float* Q1, const float* q1,
                                                        const float* Q2, const float* q2, float* zq, float* y, int64_t M) {
   constexpr int XS = kW + 4;
   extern __shared__ __align__(16) unsigned char fsm[];
