@@ -488,9 +488,14 @@ static int autotune_impl(const bdda_plan* p, int L, const T* ghat, const int32_t
   }
   for (auto& k : keys) {
     if (k.cand.empty()) continue;
+    // The default kernel stays unless another is 10 % faster: nearer ones are
+    // chosen by the noise of a run, and with them the rounding of a solve (the
+    // mixed form's iteration count moves by several).  At 192 x 224 x 350, L = 64,
+    // that keeps the two-stage complex128 X pass (15 % faster), and the complex64
+    // defaults (19.7 ms, 19.6 with the fastest of each pass).
     size_t b = 0;
     for (size_t i = 1; i < k.ms.size(); ++i)
-      if (k.ms[i] < k.ms[b]) b = i;
+      if (k.ms[i] < (b == 0 && k.cand[0].variant == 0 ? 0.9 : 1.0) * k.ms[b]) b = i;
     set_pass_tune(k.cand[b]);
   }
   if (status == BDDA_OK) {
