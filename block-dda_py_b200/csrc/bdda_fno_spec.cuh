@@ -195,12 +195,17 @@ __global__ void __launch_bounds__(256) spec_mix_bwd_data_kernel(const float2* gS
   __shared__ float2 gs[8][kWd];
   const int k = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   float2 r[kWd];
-  const float4* row = reinterpret_cast<const float4*>(R + ((int64_t)k * kWd + lane) * kWd);
+  const float2* row = R + ((int64_t)k * kWd + lane) * kWd;
+  if ((reinterpret_cast<uintptr_t>(R) & 15) == 0) {
 #pragma unroll
-  for (int o = 0; o < kWd / 2; ++o) {
-    const float4 v = row[o];
-    r[2 * o] = make_float2(v.x, -v.y);
-    r[2 * o + 1] = make_float2(v.z, -v.w);
+    for (int o = 0; o < kWd / 2; ++o) {
+      const float4 v = reinterpret_cast<const float4*>(row)[o];
+      r[2 * o] = make_float2(v.x, -v.y);
+      r[2 * o + 1] = make_float2(v.z, -v.w);
+    }
+  } else {   // parameters on an 8-byte boundary (a slice of a larger array)
+#pragma unroll
+    for (int o = 0; o < kWd; ++o) r[o] = make_float2(row[o].x, -row[o].y);
   }
   for (int b = w; b < B; b += 8) {
     __syncwarp();
