@@ -37,8 +37,8 @@ __device__ __forceinline__ void block_copy(double2* dst, const double2* src, int
 // times that, so a factorisation step is bound by the chain pivot search ->
 // division -> scaling -> update, not by its arithmetic.  These routines
 // eliminate without dividing: the rows below a pivot d become
-// (d x - c u) 2^-e, e the exponent of d.  That scales all remaining rows (and
-// right-hand sides) by the same factor d 2^-e of modulus 1 to 3, so pivots are chosen as
+// (d x - c u) 2^-e, 2^e the power of two above d.  That scales all remaining rows (and
+// right-hand sides) by the same factor d 2^-e of modulus 0.5 to 1.4, so pivots are chosen as
 // partial pivoting chooses them and the solution is the same; the only
 // divisions, by the L pivots, run side by side before the back substitution.
 // Rows are not moved: perm[k] is the pivot row of step k; every warp finds it
@@ -51,11 +51,13 @@ __device__ __forceinline__ void block_copy(double2* dst, const double2* src, int
 constexpr int kElimMax = 32;
 __host__ __device__ constexpr int elim_pitch(int ncol) { return ncol | 1; }   // odd: column reads without bank conflicts
 
-// 2^-exponent of the larger component
+// 2^-(exponent + 1) of the larger component: the scaled value lies in [1/2, 1)
+// in it, so the rows do not grow with the steps: entries up to about 1e304 at
+// 32 columns (2^-exponent, values in [1, 2), overflowed there).
 __device__ __forceinline__ double pow2_below(double2 d) {
   const int hx = __double2hiint(fabs(d.x)) >> 20, hy = __double2hiint(fabs(d.y)) >> 20;
-  const int e = min(max(max(hx, hy), 1), 2045);
-  return __hiloint2double((2046 - e) << 20, 0);
+  const int e = min(max(max(hx, hy), 1), 2044);
+  return __hiloint2double((2045 - e) << 20, 0);
 }
 __device__ __forceinline__ double2 elim_mul(double2 a, double2 b) {   // the same operations for any operands
   return make_double2(fma(a.x, b.x, -__dmul_rn(a.y, b.y)), fma(a.x, b.y, __dmul_rn(a.y, b.x)));
