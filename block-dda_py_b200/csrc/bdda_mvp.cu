@@ -58,18 +58,22 @@ static size_t pencil_smem(int M, int LT, int kind) {
 // Launch shape of the pencil passes, per precision (0 c128, 1 c64) and pass
 // kind: the shared-memory budget per CTA (the widest column tile that fits is
 // used) and the threads per CTA.  Set by bdda_tune_set.
-static size_t g_tile_smem_budget[2][3] = {{80 * 1024, 80 * 1024, 80 * 1024},
-                                          {80 * 1024, 80 * 1024, 80 * 1024}};
-static int g_threads[2][3] = {{256, 256, 256}, {256, 256, 256}};
+constexpr size_t kTileBudget = 80 * 1024;
+constexpr int kTileThreads = 256;
+static size_t g_tile_smem_budget[2][3] = {{kTileBudget, kTileBudget, kTileBudget},
+                                          {kTileBudget, kTileBudget, kTileBudget}};
+static int g_threads[2][3] = {{kTileThreads, kTileThreads, kTileThreads}, {kTileThreads, kTileThreads, kTileThreads}};
 static_assert(K_FWD == 0 && K_CONV == 1 && K_INV == 2, "tuning tables are indexed by pass kind");
 
 // Per-pass launch choices set by the autotuner (bdda_tune_pass), keyed by
 // precision, pass kind, axis length and L: the column tile width lt (0 = the
-// shared-memory budget rule) and the kernel variant (0 = the first
-// specialised kernel compiled, k > 0 = the one with that id in the tables:
-// register bound, CTA size and column pairs as bdda_fixed.cuh numbers them,
-// -1 = the generic kernel).
+// shared-memory budget rule) and the kernel variant (0 = the library's choice,
+// among the kernels of that tile width when lt is given; k > 0 = the one with
+// that id in the tables: register bound, CTA size and column pairs as
+// bdda_fixed.cuh numbers them; kLineVariant = the two-register-stage kernel of
+// the length; -1, -2 = the generic kernels).
 struct PassTune { int prec, kind, M, L, lt, variant; };
+constexpr int kLineVariant = 4096;
 static std::vector<PassTune> g_pass_tune;
 static std::mutex g_tune_mu;
 
@@ -262,12 +266,18 @@ template <typename T, int KIND>
 static int launch_pass(const PassArgs& a, int64_t P0, int lt, cudaStream_t st) {
   int variant = 0;
   if (!a.green) {
-    variant = pass_tune(prec_of<T>(), KIND, a.ax.M, a.L).variant;
-    if (variant == 0) {
-      const FixedKernel* f = prec_of<T>() == 0 ? fixed_long(KIND, a.ax) : nullptr;
-      if (f) return f->fn(a, P0, st);
+    const PassTune t = pass_tune(prec_of<T>(), KIND, a.ax.M, a.L);
+    variant = t.variant;
+    // kernels whose tile is their own: not where a tile width (bdda_tune_pass) or
+    // a launch shape (bdda_tune_set) is asked for
+    const bool open = variant == 0 && t.lt == 0 && g_tile_smem_budget[prec_of<T>()][KIND] == kTileBudget &&
+                      g_threads[prec_of<T>()][KIND] == kTileThreads;
+    const FixedKernel* own = open && prec_of<T>() == 0 ? fixed_long(KIND, a.ax) : nullptr;
+    if (own) return own->fn(a, P0, st);
+    if (open || variant == kLineVariant) {
       const LineLaunchFn line = line_find(prec_of<T>(), KIND, a);
       if (line) return line(a, P0, st);
+      variant = 0;
     }
     FixedLaunchFn f = fixed_find(prec_of<T>(), KIND, lt, a.ax, variant, pair_ok(a));
     if (f) return f(a, P0, st);
@@ -419,6 +429,7 @@ static int autotune_impl(const bdda_plan* p, int L, const T* ghat, const int32_t
     int kind, axis;
     std::vector<PassTune> cand;
     std::vector<double> ms;
+    int def;   // the candidate that runs when nothing is set (-1: not among them)
   };
   std::vector<Key> keys;
   int key_of[5];
@@ -434,18 +445,23 @@ static int autotune_impl(const bdda_plan* p, int L, const T* ghat, const int32_t
       Key key;
       key.kind = pass_kind[q];
       key.axis = pass_axis[q];
-      if (line_find(prec, key.kind, pa[q])) {   // variant 0, at any tile width
-        for (int lt : {8, 4, 2})
+      key.def = -1;
+      const FixedKernel* own = prec == 0 ? fixed_long(key.kind, pa[q].ax) : nullptr;
+      if (!own && line_find(prec, key.kind, pa[q])) {
+        key.def = 0;
+        for (int lt : {8, 4, 2})   // its tile is its own: lt only names a width that fits the other kernels
           if (pencil_smem<T>(M, lt, key.kind) <= 227 * 1024) {
-            key.cand.push_back({prec, key.kind, M, L, lt, 0});
+            key.cand.push_back({prec, key.kind, M, L, lt, kLineVariant});
             break;
           }
       }
       for (int lt : {16, 8, 4, 2}) {
         if (lt > 2 && lt / 2 >= L) continue;
         if (pencil_smem<T>(M, lt, key.kind) > 227 * 1024) continue;
-        for (int v : fixed_variants(prec, key.kind, lt, p->ax[key.axis], pair_ok(pa[q])))
+        for (int v : fixed_variants(prec, key.kind, lt, p->ax[key.axis], pair_ok(pa[q]))) {
+          if (own && own->lt == lt && own->variant == v) key.def = (int)key.cand.size();
           key.cand.push_back({prec, key.kind, M, L, lt, v});
+        }
         if (lt <= 8) {   // generic kernels go up to 8: global loads, TMA-filled tile
           key.cand.push_back({prec, key.kind, M, L, lt, -1});
           key.cand.push_back({prec, key.kind, M, L, lt, -2});
@@ -493,9 +509,9 @@ static int autotune_impl(const bdda_plan* p, int L, const T* ghat, const int32_t
     // mixed form's iteration count moves by several).  At 192 x 224 x 350, L = 64,
     // that keeps the two-stage complex128 X pass (15 % faster), and the complex64
     // defaults (19.7 ms, 19.6 with the fastest of each pass).
-    size_t b = 0;
-    for (size_t i = 1; i < k.ms.size(); ++i)
-      if (k.ms[i] < (b == 0 && k.cand[0].variant == 0 ? 0.9 : 1.0) * k.ms[b]) b = i;
+    size_t b = (size_t)std::max(k.def, 0);
+    for (size_t i = 0; i < k.ms.size(); ++i)
+      if (k.ms[i] < ((int)b == k.def ? 0.9 : 1.0) * k.ms[b]) b = i;
     set_pass_tune(k.cand[b]);
   }
   if (status == BDDA_OK) {
@@ -679,7 +695,7 @@ int bdda_tune_set(int prec, int kind, size_t smem_budget, int threads) {
 
 int bdda_tune_pass(int prec, int kind, int M, int L, int lt, int variant) {
   if (prec < 0 || prec > 1 || kind < 0 || kind > 2 || M < 1 || L < 1 || L > kMaxL ||
-      (lt != 0 && lt != 2 && lt != 4 && lt != 8 && lt != 16) || variant < -2 || variant >= 4096)
+      (lt != 0 && lt != 2 && lt != 4 && lt != 8 && lt != 16) || variant < -2 || variant > kLineVariant)
     return BDDA_BAD_ARG;
   set_pass_tune({prec, kind, M, L, lt, variant});
   return BDDA_OK;

@@ -92,15 +92,20 @@ int bdda_plan_wait_timeouts(const bdda_plan* plan, unsigned int* count, void* st
  * the autotuner).  kind: 0 forward passes (Z, Y), 1 X pass (forward, Green
  * multiply, inverse), 2 inverse passes (Y^-1, Z^-1).  smem_budget bounds the
  * shared memory of one CTA and so selects the widest column tile that fits;
- * threads per CTA is a multiple of 32 up to 512.  Process-wide settings. */
+ * threads per CTA is a multiple of 32 up to 512.  Process-wide settings.  With
+ * the initial shape (80 KiB, 256) passes run kernels whose tile is their own
+ * where there are any (variant 0 below); with any other, those of that shape. */
 int bdda_tune_set(int prec, int kind, size_t smem_budget, int threads);
 int bdda_tune_get(int prec, int kind, size_t* smem_budget, int* threads);
 /* Per-pass launch choice for passes of (prec, kind) over an axis of length M
  * at block width L: column tile width lt (2, 4, 8, 16; 0 = the smem_budget rule)
- * and kernel variant (0 = the library's choice: the two-register-stage kernel
- * of the axis length (even 7-smooth lengths from 16 to 540), except where a
+ * and kernel variant (0 = the library's choice: for lt 0 the two-register-stage
+ * kernel of the axis length, where there is one (even 7-smooth lengths from 16 to
+ * 540 without 486 and 490; X passes up to 320 without 250), except where a
  * complex128 axis of at least 192 points has kernels specialised for its radix
- * sequence; k in 1..8 = the one of 256 threads compiled for k resident CTAs
+ * sequence; for a given lt the first kernel of that tile width specialised for the
+ * radix sequence, or the generic one; 4096 = the two-register-stage kernel, whose
+ * tile is its own; k in 1..8 = the specialised kernel of 256 threads compiled for k resident CTAs
  * per SM; k + 16 * (threads / 32) = the one of that CTA size; 512 + either
  * = a complex64 kernel whose jobs take two adjacent columns, used when L is
  * even and the pass's field pointers are 16-byte aligned; 1024 + any of
@@ -125,7 +130,8 @@ int bdda_tune_pass_variants(const bdda_plan* plan, int prec, int kind, int axis,
  * itself).  Runs block MVPs of this plan on the caller's buffers (arguments as
  * bdda_block_mvp; out and work are overwritten), times each pass over every
  * candidate (tile width x kernel variant) with CUDA events, reps timed
- * products per candidate, and keeps the fastest per pass key through
+ * products per candidate, and keeps the library's own choice of a pass key, or the
+ * fastest candidate if that is over 10 % faster, through
  * bdda_tune_pass.  ms_before / ms_after (nullable): one product before and
  * after.  Synchronises the stream; do not call during stream capture. */
 int bdda_autotune(const bdda_plan* plan, int prec, int L, const void* ghat, const int32_t* cell_map,
