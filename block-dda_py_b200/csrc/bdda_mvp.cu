@@ -200,15 +200,21 @@ static std::vector<int> fixed_variants(int prec, int kind, int lt, const AxisFFT
 static const struct { int prec, kind; LineTableFn table; } kLineTables[] = {BDDA_LINE_TABLES(BDDA_LINE_ROW)};
 #undef BDDA_LINE_ROW
 
-// Long axes (M >= 192) with complex128 kernels specialised for their radix
-// sequence keep those: block BiCGSTAB amplifies a difference in a product's last
-// bits up to 1e9-fold in S_bk on particles of that size, the
-// two-register-stage kernels gain only 4 % there (192 x 224 x 350, L = 64:
-// 37.0 against 38.6 ms a product), and so such solutions stay the same bits.
-// The specialised kernel taken is the one with the widest TMA-filled tile
-// (52.8 ms with the first one compiled).
-static const FixedKernel* fixed_long(int kind, const AxisFFT& ax) {
-  if (!g_use_fixed || ax.M < 192 || ax.nst > 4) return nullptr;
+// Wide blocks on long axes (M >= 192) keep the complex128 kernels specialised for
+// their radix sequence, where there are any, so that their solutions stay the
+// same bits: block BiCGSTAB amplifies a difference in a product's last bits with
+// the width of the block.  On the 93 x 112 x 174 lattice (192 x 224 x 350) S_bk
+// of a solve to 1e-2 or 1e-5 moves by up to 2e-13 (relative) at L <= 8, 9e-11 at
+// 16, 5e-10 at 24, 4e-9 at 32, 5e-6 at 48 and 2e-7 at 64 when the two-register-stage
+// kernels take their place.  Those are faster at every width (dense product of
+// 96 x 112 x 175 cells: L = 1 4.06 -> 1.00 ms, 4 3.96 -> 2.82, 16 11.0 -> 9.7,
+// 32 22 -> 19, 64 45 -> 38; an axis of 350 alone is even from 5 columns on, and
+// 5-8 % slower at 3 and 4), so narrower blocks, which also leave the specialised
+// tiles partly empty, run them.  The specialised kernel taken is the one with the
+// widest TMA-filled tile (L = 64: 53 ms with the first one compiled).
+constexpr int kWideBlock = 32;
+static const FixedKernel* fixed_long(int kind, const AxisFFT& ax, int L) {
+  if (!g_use_fixed || L < kWideBlock || ax.M < 192 || ax.nst > 4) return nullptr;
   const FixedKernel* best = nullptr;
   for (int t = 0; t < kFixedTables; ++t) {
     int n = 0;
@@ -253,7 +259,7 @@ static LineLaunchFn line_find(int prec, int kind, const PassArgs& a) {
 
 bool mvp_line(int prec, const PassArgs a[5], LineLaunchFn fn[5]) {
   for (int q = 0; q < 5; ++q) {
-    fn[q] = prec == 0 && fixed_long(kPassKind[q], a[q].ax) ? nullptr : line_find(prec, kPassKind[q], a[q]);
+    fn[q] = prec == 0 && fixed_long(kPassKind[q], a[q].ax, a[q].L) ? nullptr : line_find(prec, kPassKind[q], a[q]);
     if (!fn[q]) return false;
   }
   return true;
@@ -272,7 +278,7 @@ static int launch_pass(const PassArgs& a, int64_t P0, int lt, cudaStream_t st) {
     // a launch shape (bdda_tune_set) is asked for
     const bool open = variant == 0 && t.lt == 0 && g_tile_smem_budget[prec_of<T>()][KIND] == kTileBudget &&
                       g_threads[prec_of<T>()][KIND] == kTileThreads;
-    const FixedKernel* own = open && prec_of<T>() == 0 ? fixed_long(KIND, a.ax) : nullptr;
+    const FixedKernel* own = open && prec_of<T>() == 0 ? fixed_long(KIND, a.ax, a.L) : nullptr;
     if (own) return own->fn(a, P0, st);
     if (open || variant == kLineVariant) {
       const LineLaunchFn line = line_find(prec_of<T>(), KIND, a);
@@ -446,7 +452,7 @@ static int autotune_impl(const bdda_plan* p, int L, const T* ghat, const int32_t
       key.kind = pass_kind[q];
       key.axis = pass_axis[q];
       key.def = -1;
-      const FixedKernel* own = prec == 0 ? fixed_long(key.kind, pa[q].ax) : nullptr;
+      const FixedKernel* own = prec == 0 ? fixed_long(key.kind, pa[q].ax, L) : nullptr;
       if (!own && line_find(prec, key.kind, pa[q])) {
         key.def = 0;
         for (int lt : {8, 4, 2})   // its tile is its own: lt only names a width that fits the other kernels
@@ -891,8 +897,9 @@ int bdda_green_build(const bdda_plan* p, double lf, double k, void* ghat, void* 
   ax.src = G; ax.src_p0 = Mz * 6; ax.src_p1 = 6; ax.src_row = My * Mz * 6;
   ax.dst = ghat; ax.dst_p0 = Mz * Mx * 6; ax.dst_p1 = Mx * 6; ax.dst_row = 6;   // x-pencil-major spectrum
   ax.mirror = 1 << 1 | 1 << 2;
-  const LineLaunchFn ly = fixed_long(K_FWD, ay.ax) ? nullptr : line_find(BDDA_C128, K_FWD, ay);
-  const LineLaunchFn lx = fixed_long(K_CONV, ax.ax) ? nullptr : line_find(BDDA_C128, K_FWD, ax);
+  // one spectrum for blocks of any width, so the rule of the wide ones
+  const LineLaunchFn ly = fixed_long(K_FWD, ay.ax, kMaxL) ? nullptr : line_find(BDDA_C128, K_FWD, ay);
+  const LineLaunchFn lx = fixed_long(K_CONV, ax.ax, kMaxL) ? nullptr : line_find(BDDA_C128, K_FWD, ax);
   const int64_t Px = lx ? Nx : Mx;
   {  // real-space tensor evaluated in the kernel, forward z
     PassArgs a = b;

@@ -103,7 +103,7 @@ int bdda_tune_get(int prec, int kind, size_t* smem_budget, int* threads);
  * kernel of the axis length, where there is one (even 7-smooth lengths from 16 to
  * 540 without 486 and 490; X passes up to 320 without 250), except where a
  * complex128 axis of at least 192 points has kernels specialised for its radix
- * sequence; for a given lt the first kernel of that tile width specialised for the
+ * sequence and L is at least 32; for a given lt the first kernel of that tile width specialised for the
  * radix sequence, or the generic one; 4096 = the two-register-stage kernel, whose
  * tile is its own; k in 1..8 = the specialised kernel of 256 threads compiled for k resident CTAs
  * per SM; k + 16 * (threads / 32) = the one of that CTA size; 512 + either

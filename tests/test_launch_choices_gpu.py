@@ -72,3 +72,20 @@ def test_a_launch_shape_selects_the_kernels_that_have_one(prec):
         for kind in range(3):
             _lib().bdda_tune_set(prec, kind, budget.value, threads.value)
     assert torch.equal(run(), own)
+
+
+@pytest.mark.parametrize("axis,M", [(0, 192), (1, 224), (2, 350)])
+def test_long_complex128_axes_specialised_kernels_from_32_columns(axis, M):
+    """Narrower blocks run the two-register-stage kernel of the length."""
+    n, m = [10, 11, 9], [20, 24, 18]
+    n[axis], m[axis] = M // 2 - 1, M
+    for L, line in ((1, True), (4, True), (31, True), (32, False), (64, False)):
+        run = _product(n, m, L, 0)
+        own = run()
+        try:
+            for kind in ((1,), (0, 2), (0, 2))[axis]:
+                assert _lib().bdda_tune_pass(0, kind, M, L, 0, LINE) == 0
+            assert torch.equal(run(), own) == line, L
+        finally:
+            for kind in range(3):
+                _lib().bdda_tune_pass(0, kind, M, L, 0, 0)
