@@ -20,16 +20,16 @@
 // M^-1 (B - A X) after every 10-fold drop (bdda_tune_mixed) and before stopping, warm
 // restarts while the true residual is above tol).
 //
-// A problem whose axes have two-register-stage kernels (every even 7-smooth
-// length up to 540, X up to 320; complex128 axes that keep their specialised
-// kernels do not) runs its five pencil passes as launches of those, skipped on
-// the device while its flag is clear; the problems' chains run side by side on
-// up to kSides streams.  The products of the other problems share launches of
-// the generic run-time-radix kernel body (problems have different radix
-// sequences), which all of them did before.  39 iterations, 32 problems of
-// 8^3 cells and 8 columns: 32.9 -> 26.2 ms; 256 of 14^3: 703 -> 365; 16 of 18^3
-// and 16 columns: 147 -> 70; one of 12^3: 9.5 -> 4.5; mixed form 45 -> 44, 674 ->
-// 460, 163 -> 101, 10.2 -> 5.8.  No size measured is better off sharing.
+// A problem whose axes all have two-register-stage kernels (even 7-smooth lengths
+// from 16 to 540 without 486 and 490, X up to 320 without 250 and 294) runs its five
+// pencil passes as launches of those, skipped on the device while its flag is
+// clear; the problems' chains run side by side on up to kSides streams.  The
+// products of the other problems share launches of the generic run-time-radix
+// kernel body (problems have different radix sequences), which all of them did
+// before.  39 iterations, 32 problems of 8^3 cells and 8 columns: 32.9 -> 26.2 ms;
+// 256 of 14^3: 703 -> 365; 16 of 18^3 and 16 columns: 147 -> 70, 8 of 32 x 32 x 112
+// 1083 -> 536; one of 12^3: 9.5 -> 4.5; mixed form 45 -> 44, 674 -> 460, 163 -> 101,
+// 10.2 -> 5.8.  No size measured is better off sharing.
 // The Gram, update and dot kernels use the
 // L-specialised bodies, so L is one of 8, 16, 32, 64.
 #include <algorithm>
@@ -56,7 +56,9 @@ constexpr int kCheckEvery = 4;    // iterations between host reads of the active
 // Iterations before the iteration's graph is built: a launch in the graph saves
 // 2 us an iteration and costs 15 us to build and release, so a batch that ends
 // within as many iterations as pay for it goes without (4 iterations of 8
-// problems of 16,000 cells: 1.5 ms of 8.5).
+// problems of 16,000 cells: 1.5 ms of 8.5).  A longer one pays for those launches:
+// 39 iterations of 32 problems of 8^3 cells 22.3 -> 26.2 ms, of 256 of 14^3 325 ->
+// 365, against a graph from the first iteration.
 constexpr int kDirect = 8;
 constexpr int kRowsPerBlasItem = 512;
 constexpr size_t kPencilBudget = 80 * 1024;

@@ -259,7 +259,7 @@ static LineLaunchFn line_find(int prec, int kind, const PassArgs& a) {
 
 bool mvp_line(int prec, const PassArgs a[5], LineLaunchFn fn[5]) {
   for (int q = 0; q < 5; ++q) {
-    fn[q] = prec == 0 && fixed_long(kPassKind[q], a[q].ax, a[q].L) ? nullptr : line_find(prec, kPassKind[q], a[q]);
+    fn[q] = line_find(prec, kPassKind[q], a[q]);
     if (!fn[q]) return false;
   }
   return true;

@@ -569,7 +569,7 @@ struct LineKernel {
   LineLaunchFn fn;
 };
 // Line kernels (bdda_line.cuh) of the five passes whose arguments a holds; false
-// if one of them has none, or keeps its specialised kernel.
+// if one of them has none.
 bool mvp_line(int prec, const PassArgs a[5], LineLaunchFn fn[5]);
 typedef const LineKernel* (*LineTableFn)(int* n);
 #define BDDA_LINE_TABLES(F)                                                                            \
