@@ -231,7 +231,19 @@ static const FixedKernel* fixed_long(int kind, const AxisFFT& ax, int L) {
   return best;
 }
 
-// Two-register-stage kernel of a pass (bdda_line.cuh), or null: the length must
+// Two-register-stage kernel of a length (bdda_line.cuh; kind 3: over mirrored rows), or null.
+static LineLaunchFn line_of(int prec, int kind, int M) {
+  for (const auto& t : kLineTables) {
+    if (t.prec != prec || t.kind != kind) continue;
+    int n = 0;
+    const LineKernel* k = t.table(&n);
+    for (int i = 0; i < n; ++i)
+      if (k[i].M == M && k[i].fn) return k[i].fn;
+  }
+  return nullptr;
+}
+
+// Two-register-stage kernel of a pass, or null: the length must
 // have a split, and the rows a product reads (forward), writes (inverse) or
 // both (X) lie in the first half of the pencil, as on any grid M >= 2 N.
 static LineLaunchFn line_find(int prec, int kind, const PassArgs& a) {
@@ -247,14 +259,7 @@ static LineLaunchFn line_find(int prec, int kind, const PassArgs& a) {
   } else {
     if (2 * a.n_in > M || 2 * a.n_out > M || a.src_p1 != a.C || a.dst_p1 != a.C || a.src_p0 != a.dst_p0) return nullptr;
   }
-  for (const auto& t : kLineTables) {
-    if (t.prec != prec || t.kind != want) continue;
-    int n = 0;
-    const LineKernel* k = t.table(&n);
-    for (int i = 0; i < n; ++i)
-      if (k[i].M == M && k[i].fn) return k[i].fn;
-  }
-  return nullptr;
+  return line_of(prec, want, M);
 }
 
 bool mvp_line(int prec, const PassArgs a[5], LineLaunchFn fn[5]) {
@@ -720,7 +725,9 @@ int bdda_tune_pass_variants(const bdda_plan* plan, int prec, int kind, int axis,
   if (!plan || !n || prec < 0 || prec > 1 || kind < 0 || kind > 2 || axis < 0 || axis > 2 || cap < 0 ||
       (cap > 0 && !variants))
     return BDDA_BAD_ARG;
-  const std::vector<int> v = fixed_variants(prec, kind, lt, plan->ax[axis], true);
+  std::vector<int> v;
+  if (lt != 0) v = fixed_variants(prec, kind, lt, plan->ax[axis], true);
+  else if (2 * plan->n[axis] <= plan->ax[axis].M && line_of(prec, kind, plan->ax[axis].M)) v.push_back(kLineVariant);
   *n = (int)v.size();
   for (int i = 0; i < (int)v.size() && i < cap; ++i) variants[i] = v[i];
   return BDDA_OK;

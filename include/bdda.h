@@ -101,7 +101,7 @@ int bdda_tune_get(int prec, int kind, size_t* smem_budget, int* threads);
  * at block width L: column tile width lt (2, 4, 8, 16; 0 = the smem_budget rule)
  * and kernel variant (0 = the library's choice: for lt 0 the two-register-stage
  * kernel of the axis length, where there is one (even 7-smooth lengths from 16 to
- * 540 without 486 and 490; X passes up to 320 without 250), except where a
+ * 540 without 486 and 490; X passes up to 320 without 250 and 294), except where a
  * complex128 axis of at least 192 points has kernels specialised for its radix
  * sequence and L is at least 32; for a given lt the first kernel of that tile width specialised for the
  * radix sequence, or the generic one; 4096 = the two-register-stage kernel, whose
@@ -123,7 +123,8 @@ int bdda_tune_pass(int prec, int kind, int M, int L, int lt, int variant);
 int bdda_tune_pass_get(int prec, int kind, int M, int L, int* lt, int* variant);
 /* Variant ids (as bdda_tune_pass) of the specialised kernels compiled for the
  * pass (prec, kind) over this plan's axis (0 = x, 1 = y, 2 = z) at tile width
- * lt: up to cap of them into variants, their number into *n. */
+ * lt (0: of the kernel whose tile is its own): up to cap of them into variants,
+ * their number into *n. */
 int bdda_tune_pass_variants(const bdda_plan* plan, int prec, int kind, int axis, int lt, int* variants, int cap,
                             int* n);
 /* Autotuner (no counterpart in the reference; the reference's scipy.fft plans
