@@ -261,24 +261,27 @@ _BATCH_KEEP_BYTES = 4 << 30
 
 
 def _batch_groups(entries, mode, L, itermax, max_bytes):
-    """Index groups of similar lattice size whose workspace fits max_bytes
-    (at most 1024 problems each), largest lattices first."""
+    """(index groups of similar lattice size whose workspace fits max_bytes, at
+    most 1024 problems each, largest lattices first; whether max_bytes set a
+    group's end)."""
     lib = _lib.load()
     size = [max(e["g"].plan.m) for e in entries]
     order = sorted(range(len(entries)), key=lambda i: -size[i])
-    groups, cur = [], []
+    groups, cur, bound = [], [], False
     for i in order:
         trial = cur + [i]
         nbytes = int(lib.bdda_batch_workspace_bytes(_batch_struct([entries[j] for j in trial], mode), len(trial),
                                                     mode, L, itermax))
-        if cur and (len(trial) > 1024 or nbytes > max_bytes or size[cur[0]] > _SIZE_RATIO * size[i]):
+        other = len(trial) > 1024 or (cur and size[cur[0]] > _SIZE_RATIO * size[i])
+        if cur and (other or nbytes > max_bytes):
+            bound = bound or not other
             groups.append(cur)
             cur = [i]
         else:
             cur = trial
     if cur:
         groups.append(cur)
-    return groups
+    return groups, bound
 
 
 def bl_bicgstab_jacobi_mvp_fft_batch(problems, tol, itermax, precision=None, max_outer=20,
@@ -329,17 +332,16 @@ def bl_bicgstab_jacobi_mvp_fft_batch(problems, tol, itermax, precision=None, max
     small = [i for i in range(len(entries)) if i not in set(big)]
     split = lambda bound: _batch_groups([entries[i] for i in small], mode, L, itermax, bound)
     if fixed_bound:
-        groups = split(max_bytes)
+        groups, _ = split(max_bytes)
     else:
         # memory that torch's allocator holds counts as free once it is given
         # back; that (and taking the workspace from the device anew) costs over a
-        # millisecond a call, so only when it decides how the batch is split
-        free, total = torch.cuda.mem_get_info(dev)
-        groups = split(int(0.7 * free))
-        if groups != split(total):
+        # millisecond a call, so only when memory decides how the batch is split
+        # (one split of 128 problems takes 7 ms: a second one is made only then)
+        groups, bound = split(int(0.7 * torch.cuda.mem_get_info(dev)[0]))
+        if bound:
             torch.cuda.empty_cache()
-            free, total = torch.cuda.mem_get_info(dev)
-            groups = split(int(0.7 * free))
+            groups, _ = split(int(0.7 * torch.cuda.mem_get_info(dev)[0]))
     groups = [[small[j] for j in g] for g in groups]
     for g in [g for g in groups if len(g) == 1]:
         big.append(g[0])
