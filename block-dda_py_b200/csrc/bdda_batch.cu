@@ -29,7 +29,7 @@
 // before.  39 iterations, 32 problems of 8^3 cells and 8 columns: 32.9 -> 26.2 ms;
 // 256 of 14^3: 703 -> 365; 16 of 18^3 and 16 columns: 147 -> 70, 8 of 32 x 32 x 112
 // 1083 -> 536; one of 12^3: 9.5 -> 4.5; mixed form 45 -> 44, 674 -> 460, 163 -> 101,
-// 10.2 -> 5.8.  No size measured is better off sharing.
+// 10.2 -> 5.8.
 // The Gram, update and dot kernels use the
 // L-specialised bodies, so L is one of 8, 16, 32, 64.
 #include <algorithm>
@@ -60,6 +60,24 @@ constexpr int kCheckEvery = 4;    // iterations between host reads of the active
 // 39 iterations of 32 problems of 8^3 cells 22.3 -> 26.2 ms, of 256 of 14^3 325 ->
 // 365, against a graph from the first iteration.
 constexpr int kDirect = 8;
+// Batches of at least kManySmall problems, all with kernels of their own and of
+// fewer values (padded grid points x columns) on average than these (by the
+// precision of the products), run the direct iterations with shared launches, and
+// each problem's own only in the graph.  A launch of its own costs the host
+// 2.6 us, ten (in the mixed form, with the replacement's, fifteen) a problem and
+// iteration, more than the shared kernels take on such sizes: 128 problems of 8^3
+// cells and 8 columns, 98 K values, 3.3 ms an iteration against 2.4, of 10^3 3.3
+// against 3.9 (complex64 3.5 against 3.0); mixed form 5.5 against 2.5 and, of 12^3,
+// 331 K values, 5.5 against 5.2.  In the graph own launches are the faster ones
+// (8^3 1.0 ms an iteration).  Eight problems are even.
+//   128 problems, 8 columns:  shared throughout  own throughout   this
+//   8^3    4 iterations          21.8 ms            26.2          21.3
+//          39                   106                 75            66
+//   8^3 mixed, 4                 22.8               36.5          22.0
+//          39                   101                120            93
+//   10^3   4                     28.5               26.2          26.1
+constexpr int kManySmall = 16;
+constexpr double kSmallValues[2] = {1 << 17, 1 << 18};   // complex128, complex64 products
 constexpr int kRowsPerBlasItem = 512;
 constexpr size_t kPencilBudget = 80 * 1024;
 constexpr int kSides = 8;
@@ -615,6 +633,7 @@ struct Engine {
     int64_t P0[5];
   };
   std::vector<Chain> chains;
+  bool chained = true;              // those run (false: a batch of small problems before its graph)
   bool shared = true;               // some problem's passes are in the work list
   cudaStream_t side[kSides - 1];    // beside st (nside of them)
   cudaEvent_t fork = nullptr, join[kSides - 1];
@@ -702,13 +721,14 @@ struct Engine {
   // site, host: 5 x nprob PassArgs, pass-major; flags: of the listed problems
   int mvp(const PassArgs* site, const PassArgs* host, const int* flags) {
     const size_t n = (size_t)nprob;
+    const int nside = chained ? this->nside : 0;
     if (nside) {
       BDDA_CUDA_TRY(cudaEventRecord(fork, st));
       for (int i = 0; i < nside; ++i) BDDA_CUDA_TRY(cudaStreamWaitEvent(side[i], fork, 0));
     }
     // st takes a share of the chains only when it has no shared passes to run
     const int lanes = nside + (shared ? 0 : 1);
-    for (size_t c = 0; c < chains.size(); ++c) {
+    for (size_t c = 0; chained && c < chains.size(); ++c) {
       const Chain& ch = chains[c];
       const int lane = lanes ? (int)(c % lanes) : nside;
       for (int q = 0; q < 5; ++q) {
@@ -941,6 +961,7 @@ int batch_run(const bdda_batch_problem* pr, int nprob, int mode, int L, double t
   // ---- host images of the descriptors and argument sites ----
   std::vector<ProbDev> hpd(np);
   std::vector<int64_t> hcnt((size_t)2 * kNCls * np, 0);
+  std::vector<char> own(2 * np, 0);   // per list: the problem's passes have kernels of their own
   std::vector<GramArgs> hgram(kGramSites * np);
   std::vector<UpdateArgs> hupd(kUpdSites * np);
   std::vector<DotArgs> hdot(np);
@@ -1029,11 +1050,12 @@ int batch_run(const bdda_batch_problem* pr, int nprob, int mode, int L, double t
         };
         if (chain && f32 && mixed) add(e32);
         else if (chain) add(e);
+        own[(size_t)list * np + i] = chain;
       }
       for (int ps = 0; ps < 5; ++ps) {
         pa[ps].ntile = (L + ltv[ps] - 1) / ltv[ps];
         hmvp[((size_t)site * 5 + ps) * np + i] = pa[ps];
-        hcnt[((size_t)list * kNCls + ps) * np + i] = chain ? 0 : P0[ps] * pa[ps].P1 * pa[ps].ntile;
+        hcnt[((size_t)list * kNCls + ps) * np + i] = P0[ps] * pa[ps].P1 * pa[ps].ntile;
       }
     };
     const bool t32 = std::is_same<T, float2>::value;
@@ -1060,8 +1082,23 @@ int batch_run(const bdda_batch_problem* pr, int nprob, int mode, int L, double t
       { ElemArgs& x = E(EL_O2Z); x.n = rows * L; x.a = Z; x.b = w + q.out32; }
     }
   }
+  double values = 0.0;
+  for (int i = 0; i < nprob; ++i) {
+    const AxisFFT* ax = pr[i].plan->ax;
+    values += 3.0 * L * ax[0].M * ax[1].M * ax[2].M / nprob;
+  }
   e.shared = e.chains.size() < np;
   e32.shared = e32.chains.size() < np;
+  const bool early = nprob >= kManySmall && !e.shared && !(mixed && e32.shared) &&
+                     values < kSmallValues[mode == BDDA_BATCH_C128 ? 0 : 1];
+  if (early) {
+    e.shared = e32.shared = true;
+    e.chained = e32.chained = false;
+  } else {   // the work lists hold the other problems' passes
+    for (size_t k = 0; k < 2 * np; ++k)
+      for (int c = 0; own[k] && c < kNCls; ++c)
+        if (c != kClsBlas) hcnt[(k / np * kNCls + c) * np + k % np] = 0;
+  }
   Sides sides;
   {
     const int nc = (int)std::max(e.chains.size(), e32.chains.size());
@@ -1076,18 +1113,20 @@ int batch_run(const bdda_batch_problem* pr, int nprob, int mode, int L, double t
   }
   // Mixed form: the complex64 passes of a chained problem read P or T and write V
   // or Z themselves (site 0 and 1, complex128); its conversions are empty.
+  std::vector<PassArgs> hown(hmvp);   // arguments of the problems' own launches
   if (mixed)
     for (const auto& ch : e32.chains) {
       const size_t i = (size_t)ch.p;
       for (int site = 0; site < 2; ++site) {
-        for (int ps = 0; ps < 5; ++ps) hmvp[((size_t)site * 5 + ps) * np + i] = hmvp[(size_t)ps * np + i];
-        PassArgs& z0 = hmvp[((size_t)site * 5 + 0) * np + i];
-        PassArgs& z1 = hmvp[((size_t)site * 5 + 4) * np + i];
+        for (int ps = 0; ps < 5; ++ps) hown[((size_t)site * 5 + ps) * np + i] = hmvp[(size_t)ps * np + i];
+        PassArgs& z0 = hown[((size_t)site * 5 + 0) * np + i];
+        PassArgs& z1 = hown[((size_t)site * 5 + 4) * np + i];
         z0.wide = z1.wide = 1;
         z0.S = z0.src = z1.S = site == 0 ? hupd[(size_t)U_P * np + i].out : hupd[(size_t)U_T * np + i].out;
         z1.dst = w + lay.p[i].vec[site == 0 ? 4 : 6];
       }
-      for (int s : {EL_P2S, EL_T2S, EL_O2V, EL_O2Z}) hel[(size_t)s * np + i].n = 0;
+      if (!early)
+        for (int s : {EL_P2S, EL_T2S, EL_O2V, EL_O2Z}) hel[(size_t)s * np + i].n = 0;
     }
   for (int list = 0; list < 2; ++list)
     for (int c = 0; c < kNCls; ++c) {
@@ -1129,7 +1168,7 @@ int batch_run(const bdda_batch_problem* pr, int nprob, int mode, int L, double t
   auto usite = [&](int s) { return dupd + (size_t)s * np; };
   auto esite = [&](int s) { return del + (size_t)s * np; };
   auto msite = [&](int s) { return dmvp + (size_t)s * 5 * np; };
-  auto hsite = [&](int s) { return hmvp.data() + (size_t)s * 5 * np; };
+  auto hsite = [&](int s) { return hown.data() + (size_t)s * 5 * np; };
 
   // the product inside the iteration: src -> dst in T, or through complex64 in the mixed form
   auto iter_mvp = [&](int site, int to32, int from32) -> int {
@@ -1193,6 +1232,10 @@ int batch_run(const bdda_batch_problem* pr, int nprob, int mode, int L, double t
   cudaGraphExec_t gexec = nullptr;
   unsigned long long per_iter = 0;
   auto capture = [&]() -> int {
+    if (early) {   // from here on with launches of their own, graph or not
+      e.shared = e32.shared = false;
+      e.chained = e32.chained = true;
+    }
     if (!use_graph || gexec) return BDDA_OK;
     const unsigned long long before = e.launches + e32.launches;
     BDDA_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
