@@ -91,9 +91,9 @@ __device__ __forceinline__ pair2 fma2(pair2 a, pair2 b, pair2 c) {
 }
 // Normal distribution function Phi(z) = erfc(-z / sqrt 2) / 2 without a branch:
 // erfc(a) = 2^q(a) for a = |z| / sqrt 2 <= 6, q a polynomial of degree 12 with
-// q(0) = 0 fitted to log2 erfc (weighted least squares, iterated to the
-// smallest largest error, 3e-9 x max(erfc, 1e-3)).  In FP32 Phi is within 6e-8,
-// as 0.5 (1 + erff) is, for 17 instructions instead of about 40 (erff runs
+// q(0) = 0 fitted to log2 erfc (weighted least squares, iterated towards the
+// smallest largest error: 4.5e-9, and 1.5e-6 x max(erfc, 1e-3)).  In FP32 Phi is
+// within 7e-8 (0.5 (1 + erff): 6.4e-8), for 17 instructions instead of about 40 (erff runs
 // both of its branches in most warps; GELU was two thirds of the projection's
 // instructions).
 __device__ __forceinline__ float2 normal_cdf(float2 z) {
@@ -134,7 +134,7 @@ __device__ __forceinline__ float2 gelu_grad(float2 z) {
 // mma.sync m16n8k8 with TF32 operands and FP32 accumulation, each product
 // split in three, a b ~ a_hi b_hi + a_hi b_lo + a_lo b_hi with a_hi = tf32(a),
 // a_lo = tf32(a - a_hi), which keeps the accuracy of FP32 (the dropped a_lo b_lo
-// term is below FP32 rounding).  The unit's accumulator is cut, not rounded (a
+// is at most 2^-22 of a product, 2^-24 typically, an FP32 rounding 2^-24).  The unit's accumulator is cut, not rounded (a
 // relative bias of -1.5e-7 after 32 columns), so each step of 8 columns starts from
 // zero and is added in FP32: error 0.9e-7 rms, an FP32 chain's is 1.0e-7.
 // Fragments of m16n8k8 (lane = 4 g + t):

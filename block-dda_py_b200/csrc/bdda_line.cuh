@@ -24,10 +24,12 @@
 //
 // Bound.  Z and Y passes: memory latency, hence small tiles, one job per
 // thread, as many CTAs as the registers allow (4.2-6.1 of the 6.56 TB/s copy
-// rate in complex128).  X pass in complex128: the FP64 pipe (58 instructions a
-// grid value, 55-60 % of its peak): a CTA works through the column tiles of one
-// pencil with the pencil's Green's entries staged once in shared memory, and
-// asks for the next tile's rows before it computes.  One product on a B200, the
+// rate in complex128).  X pass in complex128: the FP64 pipe (66 instructions a
+// grid value at 90 points, 56 % of its peak by the counters): a CTA works through
+// the column tiles of one pencil with the pencil's Green's entries staged once in
+// shared memory, and asks for the next tile's rows before it computes.  In
+// complex64: issue (69 % of the slots at 192 points) and shared memory (52 % of its
+// wavefronts).  One product on a B200, the
 // run-time-radix kernels -> these (time of the bytes at the copy rate):
 //   17 x 17 x 17    L = 10  complex128   105 -> 45 us     (11)
 //   52 x 60 x 71    L = 1   complex128   534 -> 141 us    (71)
@@ -110,7 +112,8 @@ template <typename T, int M, int KIND> struct LineShape {
 // X pass.  A middle job holds 3 B complex values, so few CTAs fit the
 // register file, and what a CTA waits for (its loads, the barriers between its
 // stages) has to be covered by the others: as many CTAs as shared memory and
-// the jobs' registers allow without spilling.
+// the jobs' registers allow.  55 of the 200 kernels spill to get there, most of them
+// 20 bytes a thread or less (the most, 168, complex64 at 200 points).
 template <typename T, int M> struct ConvShape {
   static constexpr int A = conv_split(M), B = A ? M / A : 0, H = A / 2;
   static constexpr bool C128 = sizeof(T) == 16;
@@ -583,8 +586,9 @@ constexpr LineLaunchFn conv_entry() {
   else return nullptr;
 }
 
-// The even 7-smooth lengths from 16: those up to 128, and those above (up to
-// 540, a side of 270 cells; the X pass splits up to 320).
+// The even 7-smooth lengths from 16 to 540 (a side of 270 cells) that have a split:
+// all but 486 and 490.  The X pass has kernels of the first two lists, except 250;
+// 294, in the third, has no split for it either.
 #define BDDA_LINE_SHORT(F)                                                                              \
   F(16) F(18) F(20) F(24) F(28) F(30) F(32) F(36) F(40) F(42) F(48) F(50) F(54) F(56) F(60) F(64) F(70) \
   F(72) F(80) F(84) F(90) F(96) F(98) F(100) F(108) F(112) F(120) F(126) F(128)

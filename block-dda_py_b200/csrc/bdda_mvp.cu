@@ -515,11 +515,14 @@ static int autotune_impl(const bdda_plan* p, int L, const T* ghat, const int32_t
   }
   for (auto& k : keys) {
     if (k.cand.empty()) continue;
-    // The default kernel stays unless another is 10 % faster: nearer ones are
-    // chosen by the noise of a run, and with them the rounding of a solve (the
-    // mixed form's iteration count moves by several).  At 192 x 224 x 350, L = 64,
-    // that keeps the two-stage complex128 X pass (15 % faster), and the complex64
-    // defaults (19.7 ms, 19.6 with the fastest of each pass).
+    // The default kernel stays unless another is 10 % faster: nearer ones would be
+    // chosen by the noise of a run, and with them the last bits of a solve.  At
+    // 192 x 224 x 350, L = 64, that takes the other two-stage kernel for the
+    // complex128 X pass (15 % faster, 41.5 -> 39.0 ms a product) and the column-pair
+    // kernel for the complex64 Z^-1 pass (18 %, 20.1 -> 19.7).  The choice moves the
+    // mixed form's iteration count on one orientation set by several (22 to 28 on
+    // one, 22 to 42 on another), not on average: 60 sets 24.0 +- 0.5 with the
+    // defaults, 23.4 +- 0.4 with these.
     size_t b = (size_t)std::max(k.def, 0);
     for (size_t i = 0; i < k.ms.size(); ++i)
       if (k.ms[i] < ((int)b == k.def ? 0.9 : 1.0) * k.ms[b]) b = i;
