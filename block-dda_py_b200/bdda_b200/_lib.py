@@ -63,6 +63,7 @@ PROTOTYPES = {
     "bdda_mixed_solve": (_i, [_vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _d, _i, _i, _vp, _pi, _pd, _pd,
                               _vp, _sz, _vp]),
     "bdda_batch_bicgstab": (_i, [_vp, _i, _i, _i, _d, _i, _i, _i, _pi, _pi, _pd, _pd, _vp, _sz, _vp]),
+    "bdda_tune_choose": (_i, [_i, _pi, _pi, _pd, _pi]),
     "bdda_tune_pass_get": (_i, [_i, _i, _i, _i, _pi, _pi]),
     "bdda_tune_pass_variants": (_i, [_vp, _i, _i, _i, _i, _pi, _i, _pi]),
     "bdda_autotune": (_i, [_vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _pd, _pd, _vp]),

@@ -513,21 +513,17 @@ static int autotune_impl(const bdda_plan* p, int L, const T* ghat, const int32_t
       if (r < k.cand.size()) k.ms[r] += pm[q];
     }
   }
-  for (auto& k : keys) {
-    if (k.cand.empty()) continue;
-    // The default kernel stays unless another is 10 % faster: nearer ones would be
-    // chosen by the noise of a run, and with them the last bits of a solve.  At
-    // 192 x 224 x 350, L = 64, that takes the other two-stage kernel for the
-    // complex128 X pass (15 % faster, 41.5 -> 39.0 ms a product) and the column-pair
-    // kernel for the complex64 Z^-1 pass (18 %, 20.1 -> 19.7).  The choice moves the
-    // mixed form's iteration count on one orientation set by several (22 to 28 on
-    // one, 22 to 42 on another), not on average: 60 sets 24.0 +- 0.5 with the
-    // defaults, 23.4 +- 0.4 with these.
-    size_t b = (size_t)std::max(k.def, 0);
-    for (size_t i = 0; i < k.ms.size(); ++i)
-      if (k.ms[i] < ((int)b == k.def ? 0.9 : 1.0) * k.ms[b]) b = i;
-    set_pass_tune(k.cand[b]);
+  std::vector<double> ms;
+  std::vector<int> count, def, chosen(keys.size());
+  for (const auto& k : keys) {
+    ms.insert(ms.end(), k.ms.begin(), k.ms.end());
+    count.push_back((int)k.cand.size());
+    def.push_back(k.def);
   }
+  if (status == BDDA_OK) status = bdda_tune_choose((int)keys.size(), count.data(), def.data(), ms.data(), chosen.data());
+  for (size_t i = 0; i < keys.size(); ++i)   // after a failure: nothing set
+    if (status != BDDA_OK) set_pass_tune({prec, keys[i].kind, p->ax[keys[i].axis].M, L, 0, 0});
+    else if (chosen[i] >= 0) set_pass_tune(keys[i].cand[chosen[i]]);
   if (status == BDDA_OK) {
     status = timed(pm);
     if (status == BDDA_OK && ms_after) *ms_after = pm[0] + pm[1] + pm[2] + pm[3] + pm[4];
@@ -733,6 +729,39 @@ int bdda_tune_pass_variants(const bdda_plan* plan, int prec, int kind, int axis,
   else if (2 * plan->n[axis] <= plan->ax[axis].M && line_of(prec, kind, plan->ax[axis].M)) v.push_back(kLineVariant);
   *n = (int)v.size();
   for (int i = 0; i < (int)v.size() && i < cap; ++i) variants[i] = v[i];
+  return BDDA_OK;
+}
+
+// Between near equals the noise of a run would choose, and with the kernels the
+// last bits of a solve.  So the default of a pass stays unless another candidate
+// is over 10 % faster, of those the first within 3 % of the fastest is taken, and
+// the defaults stay altogether unless the changes save 5 % of the product.  At
+// 192 x 224 x 350, L = 64: complex128 X pass 21.2 -> 17.8 ms of a product of 41.5
+// (taken); complex64 Z^-1 pass 2.34 -> 2.01 of 20.0, where the next candidate takes
+// 2.02 (not taken).  The choice moves the mixed form's iteration count on one
+// orientation set by several (22 to 28 on one, 22 to 42 on another), not on average:
+// 60 sets 24.0 +- 0.5 with the defaults, 23.4 +- 0.4 with the faster Z^-1 pass.
+int bdda_tune_choose(int keys, const int* count, const int* def, const double* ms, int* chosen) {
+  if (keys < 0 || (keys > 0 && (!count || !def || !ms || !chosen))) return BDDA_BAD_ARG;
+  double before = 0.0, after = 0.0;
+  for (int k = 0; k < keys; ms += count[k++]) {
+    if (count[k] < 0 || def[k] >= count[k]) return BDDA_BAD_ARG;
+    chosen[k] = count[k] > 0 ? 0 : -1;
+    if (count[k] == 0) continue;
+    const double fastest = *std::min_element(ms, ms + count[k]);
+    if (def[k] >= 0 && !(fastest < 0.9 * ms[def[k]])) {
+      chosen[k] = def[k];
+    } else {
+      while (chosen[k] + 1 < count[k] && !(ms[chosen[k]] <= 1.03 * fastest)) ++chosen[k];
+    }
+    if (def[k] >= 0) {
+      before += ms[def[k]];
+      after += ms[chosen[k]];
+    }
+  }
+  if (!(after < 0.95 * before))
+    for (int k = 0; k < keys; ++k)
+      if (def[k] >= 0) chosen[k] = def[k];
   return BDDA_OK;
 }
 

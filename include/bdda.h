@@ -131,13 +131,19 @@ int bdda_tune_pass_variants(const bdda_plan* plan, int prec, int kind, int axis,
  * itself).  Runs block MVPs of this plan on the caller's buffers (arguments as
  * bdda_block_mvp; out and work are overwritten), times each pass over every
  * candidate (tile width x kernel variant) with CUDA events, reps timed
- * products per candidate, and keeps the library's own choice of a pass key, or the
- * fastest candidate if that is over 10 % faster, through
- * bdda_tune_pass.  ms_before / ms_after (nullable): one product before and
+ * products per candidate, and sets the candidates that bdda_tune_choose picks
+ * through bdda_tune_pass.  ms_before / ms_after (nullable): one product before and
  * after.  Synchronises the stream; do not call during stream capture. */
 int bdda_autotune(const bdda_plan* plan, int prec, int L, const void* ghat, const int32_t* cell_map,
                   const void* diag, const void* jpre, const void* S, void* out, void* work, int reps,
                   double* ms_before, double* ms_after, void* stream);
+/* The rule by which bdda_autotune picks (host only): for each of `keys` pass keys
+ * count[k] candidate times, one key after another in ms; def[k] = the candidate
+ * that the library runs when nothing is set, or -1.  chosen[k] = the default,
+ * unless another is over 10 % faster and all such changes together save 5 % of
+ * the keys with a default; else, and without a default, the first candidate within
+ * 3 % of the fastest; -1 for a key without candidates. */
+int bdda_tune_choose(int keys, const int* count, const int* def, const double* ms, int* chosen);
 /* on != 0 (default): radix sequences and block widths L with a compile-time-
  * specialised kernel use it (FFT passes, Gram products, block updates) */
 int bdda_tune_fixed(int on);
