@@ -740,7 +740,7 @@ int bdda_tune_pass_variants(const bdda_plan* plan, int prec, int kind, int axis,
 // (taken); complex64 Z^-1 pass 2.34 -> 2.01 of 20.0, where the next candidate takes
 // 2.02 (not taken).  The choice moves the mixed form's iteration count on one
 // orientation set by several (22 to 28 on one, 22 to 42 on another), not on average:
-// 60 sets 24.0 +- 0.5 with the defaults, 23.4 +- 0.4 with the faster Z^-1 pass.
+// 60 sets 23.1 +- 0.4 as chosen here, 23.4 +- 0.4 with the faster Z^-1 pass.
 int bdda_tune_choose(int keys, const int* count, const int* def, const double* ms, int* chosen) {
   if (keys < 0 || (keys > 0 && (!count || !def || !ms || !chosen))) return BDDA_BAD_ARG;
   double before = 0.0, after = 0.0;
