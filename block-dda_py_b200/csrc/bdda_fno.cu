@@ -1102,8 +1102,11 @@ template <int MD> struct Spectral {
       float2* gS = at<float2>(x, x.wl.gS);
       float2* gA = at<float2>(x, x.wl.gA);
       BDDA_TRY_F(dft_fwd(x, gz, gS, inv));
-      spec_mix_bwd_data_kernel<<<x.s.K, 256, 0, x.st>>>(gS, reinterpret_cast<const float2*>(P + x.pl.R[l]), gA, x.s.B,
-                                                        x.s.K);
+      const float2* R = reinterpret_cast<const float2*>(P + x.pl.R[l]);
+      if ((reinterpret_cast<uintptr_t>(R) & 15) == 0)
+        spec_mix_bwd_data_kernel<true><<<x.s.K, 256, 0, x.st>>>(gS, R, gA, x.s.B, x.s.K);
+      else
+        spec_mix_bwd_data_kernel<false><<<x.s.K, 256, 0, x.st>>>(gS, R, gA, x.s.B, x.s.K);
       spec_mix_bwd_weight_kernel<<<x.s.K, 256, 0, x.st>>>(at<float2>(x, x.wl.A[l]), gS,
                                                           reinterpret_cast<float2*>(G + x.pl.R[l]), x.s.B, x.s.K);
       count_launch(2);
